@@ -69,7 +69,10 @@ typedef struct {
     const int32_t *rec_ij;  /* host, nrec x 2 */
 } rtm_shot;
 
-/* Kernel launch shape (autotuned by the Python layer; 0 = default). */
+/* Kernel launch shape (autotuned by the Python layer).  With NULL, or vec, rows,
+ * warps and tsteps 0 and prefetch <= 0, the library chooses: a wavefield that
+ * fits on the chip stays there (rtm_plan_resident), others stream with a shape
+ * that follows from the grid.  Results do not depend on any of it. */
 typedef struct {
     int vec;        /* columns per lane: 1, 2 or 4 */
     int rows;       /* rows per warp task (the tasks a launch dispatches last get half as many) */
@@ -84,7 +87,8 @@ typedef struct {
                        while its pointers and schedule stay the same; 0 = direct launches */
     int tsteps;     /* time steps per launch of rtm_forward, rtm_backward and the
                        checkpointed entry points: 2 = temporal blocking (needs vec 2 or 4;
-                       bit-identical results), 1 or 0 = one step per launch */
+                       bit-identical results), 1 = one step per launch, 0 = one step when another
+                       field is set, else the library's choice */
 } rtm_tune;
 
 /* Create a plan for nshots shots on one grid: validates geometry, builds the
@@ -94,6 +98,13 @@ typedef struct {
 int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots,
                     const rtm_tune *tune, rtm_plan **out);
 int rtm_plan_destroy(rtm_plan *plan);
+
+/* 1 when the plan keeps its wavefield on the chip: one launch (or a few, when
+ * its shots do not all fit at once) then runs a whole time loop.  The plan
+ * chooses it at creation when rtm_tune leaves the launch shape to the library
+ * (NULL, or vec, rows, warps and tsteps 0 and prefetch <= 0) and every shot's
+ * window fits; results do not depend on it. */
+int rtm_plan_resident(const rtm_plan *plan);
 
 /* Floats per padded row of the internal layout (row i at (i+1)*pitch + 4). */
 int rtm_plan_pitch(const rtm_plan *plan);

@@ -69,6 +69,7 @@ def lib():
     _sig(L, "rtm_plan_create", c_int, ctypes.POINTER(RtmGrid), c_int, ctypes.POINTER(RtmShot),
          ctypes.POINTER(RtmTune), ctypes.POINTER(vp))
     _sig(L, "rtm_plan_destroy", c_int, vp)
+    _sig(L, "rtm_plan_resident", c_int, vp)
     _sig(L, "rtm_plan_pitch", c_int, vp)
     _sig(L, "rtm_plan_snapshot_floats", c_size, vp, c_int)
     _sig(L, "rtm_plan_launch_count", ctypes.c_longlong, vp)

@@ -41,7 +41,9 @@ class BatchedRTM:
     shots        : ShotGeometry list (window rows and LOCAL source/receiver
                    grid indices).
     modes        : PSV, SH or BOTH (default PSV).
-    tune         : launch shape dict, "auto" (autotuner, cached), or None.
+    tune         : launch shape dict, "auto" (the library's choice where the
+                   shots' wavefields fit on the chip, else the autotuner,
+                   cached), or None (the library's choice).
     """
 
     def __init__(self, mu, lam, rho, dx, dz, fs, nt, absorbing_frame, shots: Sequence[ShotGeometry],
@@ -55,11 +57,19 @@ class BatchedRTM:
         self.shots: List[ShotGeometry] = list(shots)
         self._model = [to_tensor(x, torch.float32, self.device) for x in (mu, lam, rho)]
         self._surface = None if surface is None else to_tensor(surface, torch.float32, self.device)
-        if tune == "auto":
-            tune = autotune.best_shape(self._make_plan, self.nz, self.shots, self.modes, self.nt)
         # time loops replayed as CUDA graphs: repeated calls on the same buffers
         # skip the per-step launch overhead
-        tune = dict(tune or {}, graphs=int(bool(graphs)))
+        graphs = int(bool(graphs))
+        if tune == "auto":
+            # shots that fit on the chip need no launch shape (the library's
+            # choice, rtm_plan_resident); others are timed
+            self.tune = dict(graphs=graphs)
+            self.plan = self._make_plan(self.tune, self.nt)
+            if self.plan.resident():
+                return
+            self.plan.close()
+            tune = autotune.best_shape(self._make_plan, self.nz, self.shots, self.modes, self.nt)
+        tune = dict(tune or {}, graphs=graphs)
         self.tune = tune
         self.plan = self._make_plan(tune, self.nt)
 

@@ -19,6 +19,7 @@
 #include "step2_kernels.cuh"
 #include "adjoint2_kernels.cuh"
 #include "plan_host.h"
+#include "resident_kernels.cuh"
 #include "step_kernels.cuh"
 
 using namespace rtm;
@@ -115,6 +116,21 @@ struct rtm_plan {
     void *cb_user = nullptr;
     int cb_every = 0;
     int live = -1;
+    // Resident propagation (resident_kernels.cuh): the tile layout chosen at
+    // plan creation, or r == 0 when the plan streams its wavefield.
+    struct Resident {
+        int r = 0, warps = 0;
+        bool surface = false;   // laid out with room for a topography mask
+        int max_src = 0, max_rec_all = 0, max_rec = 0;  // point entries per tile: sources, receivers, owned receivers
+        int4 *d_tiles = nullptr, *d_shot_tiles = nullptr;
+        int *d_sync = nullptr;   // checks passed per shot
+        uint4 *d_box = nullptr;  // outboxes of the largest launch
+        size_t box_bytes = 0;
+        std::vector<int2> waves;  // (first tile, tiles) of each launch
+    } res;
+    bool auto_shape = false;  // the launch shape is the library's choice
+    std::vector<int> src_ptr_h, rec_ptr_h;  // host copies of the row tables
+    std::vector<int2> src_ent_h, rec_ent_h;
 };
 
 namespace {
@@ -146,6 +162,7 @@ void plan_free(rtm_plan *p) {
     F(p->d_surface); F(p->d_sponge);
     for (int c = 0; c < 3; ++c) { F(p->d_img[c]); F(p->d_imgc[c]); }
     F(p->d_seis_t); F(p->d_obs_t); F(p->d_flags); F(p->d_fail_seq); F(p->d_scratch);
+    F(p->res.d_tiles); F(p->res.d_shot_tiles); F(p->res.d_sync); F(p->res.d_box);
     for (auto *gc : {&p->g_fwd, &p->g_bwd, &p->g_ckpt})
         if (gc->exec) cudaGraphExecDestroy(gc->exec);
     if (p->ev_in) cudaEventDestroy(p->ev_in);
@@ -199,8 +216,9 @@ struct BoundsScope {
         add(p->d_rec_ptr, p->n_rec_ptr * sizeof(int));
         add(p->d_src_ent, p->n_src_ent * sizeof(int2));
         add(p->d_rec_ent, p->n_rec_ent * sizeof(int2));
-        add(p->d_flags, p->nshots * sizeof(int));
+        add(p->d_flags, (p->nshots + 1) * sizeof(int));
         add(p->d_fail_seq, p->nshots * sizeof(int));
+        add(p->res.d_box, p->res.box_bytes);
         add(p->d_sponge, (size_t)std::max(p->g.absorbing_frame, 1) * F);
         for (int b = 0; b < 2; ++b)
             for (int f = 0; f < NFIELD; ++f) add(p->d_state[b][f], p->state_floats * F);
@@ -476,13 +494,276 @@ void fill_common(const rtm_plan *p, StepParams &sp) {
     sp.snap_k = -1;
 }
 
+int zero_status(rtm_plan *p, cudaStream_t s) {
+    CUDA_TRY(cudaMemsetAsync(p->d_flags, 0, (p->nshots + 1) * sizeof(int), s));
+    CUDA_TRY(cudaMemsetAsync(p->d_fail_seq, 0x7f, p->nshots * sizeof(int), s));  // 0x7f7f7f7f: none
+    return 0;
+}
 int zero_state(rtm_plan *p, cudaStream_t s) {
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < NFIELD; ++f)
             if (p->d_state[b][f])
                 CUDA_TRY(cudaMemsetAsync(p->d_state[b][f], 0, p->state_floats * sizeof(float), s));
-    CUDA_TRY(cudaMemsetAsync(p->d_flags, 0, p->nshots * sizeof(int), s));
-    CUDA_TRY(cudaMemsetAsync(p->d_fail_seq, 0x7f, p->nshots * sizeof(int), s));  // 0x7f7f7f7f: none
+    return zero_status(p, s);
+}
+
+// The per-shot status codes to host memory (synchronises), and the resident
+// kernel's error word behind them.
+int read_status(rtm_plan *p, int32_t *flags, cudaStream_t s) {
+    std::vector<int> h(p->nshots + 1);
+    CUDA_TRY(cudaMemcpyAsync(h.data(), p->d_flags, h.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    std::copy(h.begin(), h.begin() + p->nshots, flags);
+    if (h[p->nshots]) return fail(RTM_E_CUDA, "resident propagation: a wait between tiles ran out");
+    return 0;
+}
+
+// ---- resident propagation (resident_kernels.cuh)
+
+// Tile layouts and the time of one step (us, mean of the two directions, 200 to
+// 600 steps of one source and a receiver on every row, measured) with 1, 2, ...
+// of their CTAs on every SM.  Few rows per lane finish a step soonest; many keep
+// more cells on the chip and recompute a smaller share of halo.  Layouts that
+// another one beats at every size are not built (P-SV R 4 x 8 warps: 432 CTAs
+// hold 581,000 cells at 3.7 us, R 6 x 8: 288 hold 645,000 at 3.3; R 3 x 16 is
+// 5 % behind R 6 x 8).
+struct ResLayout {
+    int mode, r, warps;
+    float us[4];
+};
+constexpr ResLayout RES_LAYOUTS[] = {
+    {RTM_PSV, 2, 8, {1.05f, 1.37f, 1.78f, 2.25f}}, {RTM_PSV, 2, 12, {1.31f, 1.90f}}, {RTM_PSV, 6, 8, {2.15f, 3.30f}},
+    {RTM_SH, 2, 8, {0.85f, 1.03f, 1.23f, 1.50f}},  {RTM_SH, 4, 8, {1.20f, 1.55f, 1.85f, 2.35f}}, {RTM_SH, 8, 8, {1.53f, 2.17f}},
+    {RTM_BOTH, 2, 8, {1.85f, 2.70f, 3.75f}},       {RTM_BOTH, 2, 16, {2.20f}},       {RTM_BOTH, 4, 8, {2.90f, 4.30f}},
+};
+// Time of one step of the streaming kernels at their tuned shapes (us): small
+// grids are bound by the launch (one per two steps), large ones by issue.
+double streaming_us(int modes, long long cells) {
+    return 3.5 + (double)cells / (modes == RTM_PSV ? 170e3 : modes == RTM_SH ? 250e3 : 105e3);
+}
+
+// Calls f(dir, mode, R, NW) tags for a tile layout that exists; false else.
+template <int DIR, typename F>
+bool res_dispatch(int mode, int r, int warps, F &&f) {
+#define RES_CASE(M, RR, NN)                                                                                  \
+    if (mode == M && r == RR && warps == NN) {                                                               \
+        f(std::integral_constant<int, DIR>{}, std::integral_constant<int, M>{}, std::integral_constant<int, RR>{}, \
+          std::integral_constant<int, NN>{});                                                                \
+        return true;                                                                                         \
+    }
+    RES_CASE(RTM_PSV, 2, 8) RES_CASE(RTM_PSV, 2, 12) RES_CASE(RTM_PSV, 6, 8)
+    RES_CASE(RTM_SH, 2, 8) RES_CASE(RTM_SH, 4, 8) RES_CASE(RTM_SH, 8, 8)
+    RES_CASE(RTM_BOTH, 2, 8) RES_CASE(RTM_BOTH, 2, 16) RES_CASE(RTM_BOTH, 4, 8)
+#undef RES_CASE
+    return false;
+}
+
+size_t resident_smem(const rtm_plan *p, int r, int warps, int max_inj, int max_rec, bool surface, size_t *box = nullptr) {
+    size_t n = 0;
+    res_dispatch<0>(p->g.modes, r, warps, [&](auto, auto m, auto rr, auto nn) {
+        using L = ResSmem<decltype(m)::value, decltype(rr)::value, decltype(nn)::value>;
+        n = L::bytes(surface, max_inj, max_rec);
+        if (box) *box = 2 * (size_t)L::BOX * sizeof(uint4);
+    });
+    return n;
+}
+
+// Exchange blocks of the loop it0 .. it1-1, as the kernel cuts it.
+int resident_blocks(int it0, int it1, int ci) {
+    int n = 0;
+    for (int it = it0; it < it1; ++n) {
+        int k = std::min(RES_HALO, it1 - it);
+        if (ci > 0) k = std::min(k, (ci - it % ci) % ci + 1);
+        it += k;
+    }
+    return n;
+}
+
+void resident_params(const rtm_plan *p, ResParams &rp, int dir) {
+    std::memset(&rp, 0, sizeof rp);
+    StepParams sp;
+    fill_common(p, sp);
+    auto pair = [](float x) {
+        unsigned u;
+        std::memcpy(&u, &x, 4);
+        return ((unsigned long long)u << 32) | u;
+    };
+    rp.nz = sp.nz;
+    rp.pitch = sp.pitch;
+    rp.nt = sp.nt;
+    rp.fw = sp.fw;
+    rp.src_factor = sp.src_factor;
+    rp.idx2 = pair(sp.inv_dx);
+    rp.idz2 = pair(sp.inv_dz);
+    rp.dt2 = pair(sp.dt);
+    rp.sdt2 = pair(dir == 0 ? sp.dt : -sp.dt);
+    rp.nz2 = pair(-0.0f);
+    rp.sponge = sp.sponge;
+    rp.shots = sp.shots;
+    for (int m = 0; m < NMAT; ++m) rp.mat[m] = sp.mat[m];
+    rp.surface = sp.surface;
+    rp.src_ptr = sp.src_ptr;
+    rp.src_ent = sp.src_ent;
+    rp.rec_ptr = sp.rec_ptr;
+    rp.rec_ent = sp.rec_ent;
+    rp.nrec_total = sp.nrec_total;
+    rp.flags = p->d_flags;
+    rp.fail_seq = p->d_fail_seq;
+    rp.err = p->d_flags + p->nshots;
+    for (int f = 0; f < NFIELD; ++f) rp.store[f] = p->d_state[0][f];
+    rp.tiles = p->res.d_tiles;
+    rp.shot_tiles = p->res.d_shot_tiles;
+    rp.outbox = p->res.d_box;
+    rp.arrive = p->res.d_sync;
+    rp.max_inj = dir == 0 ? p->res.max_src : p->res.max_rec_all;
+    rp.max_rec = dir == 0 ? p->res.max_rec : 0;
+}
+
+// Run the loop of rp for every shot, wave by wave.
+int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
+    CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
+    CUDA_TRY(cudaMemsetAsync(p->res.d_box, 0, p->res.box_bytes, s));  // no packet carries tag 0
+    rp.tag0 = 0;
+    const unsigned blocks = (unsigned)resident_blocks(rp.it0, rp.it1, rp.check_interval);
+    const size_t smem = resident_smem(p, p->res.r, p->res.warps, rp.max_inj, rp.max_rec, p->res.surface);
+    for (const int2 &w : p->res.waves) {
+        rp.tile0 = w.x;
+        cudaError_t e = cudaErrorInvalidValue;
+        auto go = [&](auto d, auto m, auto r, auto n) {
+            void *args[] = {&rp};
+            auto *k = resident_kernel<decltype(d)::value, decltype(m)::value, decltype(r)::value, decltype(n)::value>;
+            e = cudaLaunchCooperativeKernel((const void *)k, dim3(w.y), dim3(32 * p->res.warps), args, smem, s);
+        };
+        if (dir == 0) res_dispatch<0>(p->g.modes, p->res.r, p->res.warps, go);
+        else res_dispatch<1>(p->g.modes, p->res.r, p->res.warps, go);
+        CUDA_TRY(e);
+        ++p->launches;
+        rp.tag0 += blocks;
+    }
+    return 0;
+}
+
+// Choose the layout in which every shot's tiles are resident together and the
+// estimated step is shortest, and build its tables.  Leaves p->res.r at 0 when
+// there is none, or when streaming is estimated to be faster.
+int resident_setup(rtm_plan *p, bool surface) {
+    const std::vector<int> &src_ptr = p->src_ptr_h, &rec_ptr = p->rec_ptr_h;
+    const std::vector<int2> &src_ent = p->src_ent_h, &rec_ent = p->rec_ent_h;
+    for (void *q : {(void *)p->res.d_tiles, (void *)p->res.d_shot_tiles, (void *)p->res.d_sync, (void *)p->res.d_box})
+        if (q) cudaFree(q);
+    p->res = rtm_plan::Resident();
+    p->res.surface = surface;
+    int dev = 0, sms = 0, coop = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return 0;
+    constexpr int ow = RES_COLS - 2 * RES_HALO;
+    const int ntz = (p->g.nz + ow - 1) / ow;
+    rtm_plan::Resident best;
+    std::vector<int4> tiles, stiles;
+    double best_us = streaming_us(p->g.modes, p->rows_total * p->g.nz);
+    for (const ResLayout &lay : RES_LAYOUTS) {
+        if (lay.mode != p->g.modes) continue;
+        const int r = lay.r, warps = lay.warps, oh = warps * r - 2 * RES_HALO;
+        // tiles of every shot; point entries of the fullest tile
+        std::vector<int4> st;
+        int max_src = 0, max_rec_all = 0, max_rec = 0, most = 0;
+        for (int s = 0; s < p->nshots; ++s) {
+            const ShotDev &d = p->shots_h[s];
+            const int ntx = (d.nx + oh - 1) / oh;
+            st.push_back(make_int4(0, ntx, ntz, 0));
+            most = std::max(most, ntx * ntz);
+            auto count = [&](const std::vector<int> &ptr, const std::vector<int2> &ent, int base, int ring) {
+                std::vector<int> n((size_t)ntx * ntz, 0);
+                for (int i = 0; i < d.nx; ++i)
+                    for (int e = ptr[base + i]; e < ptr[base + i + 1]; ++e)
+                        for (int a = std::max(0, (i - ring) / oh); a <= std::min(ntx - 1, (i + ring) / oh); ++a)
+                            for (int b = std::max(0, (ent[e].x - ring) / ow); b <= std::min(ntz - 1, (ent[e].x + ring) / ow); ++b)
+                                ++n[(size_t)a * ntz + b];
+                return *std::max_element(n.begin(), n.end());
+            };
+            max_src = std::max(max_src, count(src_ptr, src_ent, d.src_row0, RES_HALO));
+            max_rec_all = std::max(max_rec_all, count(rec_ptr, rec_ent, d.rec_row0, RES_HALO));
+            max_rec = std::max(max_rec, count(rec_ptr, rec_ent, d.rec_row0, 0));
+        }
+        // CTAs per SM: the smaller of the two directions'
+        int ctas = 0;
+        cudaError_t e = cudaSuccess;
+        for (int dir = 0; dir < 2; ++dir) {
+            const size_t smem = resident_smem(p, r, warps, dir == 0 ? max_src : max_rec_all, dir == 0 ? max_rec : 0, surface);
+            int c = 0;
+            auto query = [&](auto dd, auto m, auto rr, auto nn) {
+                auto *k = resident_kernel<decltype(dd)::value, decltype(m)::value, decltype(rr)::value, decltype(nn)::value>;
+                // the limit is the kernel's, not the plan's: always the largest
+                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, 32 * warps, smem);
+            };
+            if (smem <= 227 * 1024) {
+                if (dir == 0) res_dispatch<0>(p->g.modes, r, warps, query);
+                else res_dispatch<1>(p->g.modes, r, warps, query);
+            }
+            if (e != cudaSuccess) c = 0;
+            ctas = dir == 0 ? c : std::min(ctas, c);
+        }
+        if (e != cudaSuccess) cudaGetLastError();
+        ctas = std::min(ctas, 4);
+        while (ctas > 0 && lay.us[ctas - 1] <= 0.f) --ctas;
+        const int capacity = ctas * sms;
+        if (most > capacity || max_rec_all > RES_MAX_POINTS) continue;
+        // launches: shots by decreasing tile count, each into the first one with room
+        auto ntiles = [&](int s) { return st[s].y * st[s].z; };
+        std::vector<int> order(p->nshots);
+        for (int s = 0; s < p->nshots; ++s) order[s] = s;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ntiles(a) > ntiles(b); });
+        std::vector<std::vector<int>> bins;
+        std::vector<int> room;
+        for (int s : order) {
+            size_t b = 0;
+            while (b < bins.size() && room[b] < ntiles(s)) ++b;
+            if (b == bins.size()) {
+                bins.push_back({});
+                room.push_back(capacity);
+            }
+            bins[b].push_back(s);
+            room[b] -= ntiles(s);
+        }
+        double us = 0;
+        for (int left : room) us += lay.us[(capacity - left + sms - 1) / sms - 1];
+        if (us >= best_us) continue;
+        best_us = us;
+        best = rtm_plan::Resident();
+        tiles.clear();
+        for (auto &bin : bins) {
+            const int t0 = (int)tiles.size();
+            for (int s : bin) {
+                st[s].x = (int)tiles.size();
+                for (int a = 0; a < st[s].y; ++a)
+                    for (int b = 0; b < ntz; ++b) tiles.push_back(make_int4(s, a * oh, b * ow, a * ntz + b));
+            }
+            best.waves.push_back(make_int2(t0, (int)tiles.size() - t0));
+        }
+        stiles = std::move(st);
+        best.r = r;
+        best.warps = warps;
+        best.max_src = max_src;
+        best.max_rec_all = max_rec_all;
+        best.max_rec = max_rec;
+    }
+    if (!best.r) return 0;
+    best.surface = surface;
+    p->res = best;
+    size_t box = 0;
+    resident_smem(p, best.r, best.warps, 0, 0, false, &box);
+    int wide = 0;
+    for (const int2 &w : best.waves) wide = std::max(wide, w.y);
+    p->res.box_bytes = box * wide;
+    if (int rc = dalloc(&p->res.d_tiles, tiles.size())) return rc;
+    if (int rc = dalloc(&p->res.d_shot_tiles, stiles.size())) return rc;
+    if (int rc = dalloc(&p->res.d_sync, (size_t)p->nshots)) return rc;
+    if (int rc = dalloc(&p->res.d_box, p->res.box_bytes / sizeof(uint4))) return rc;
+    CUDA_TRY(cudaMemcpy(p->res.d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(p->res.d_shot_tiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return 0;
 }
 
@@ -547,6 +828,23 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
             }
             p->tsteps = 2;
         }
+    }
+    p->auto_shape = !tune || (tune->vec <= 0 && tune->rows <= 0 && tune->warps <= 0 && tune->tsteps == 0 && tune->prefetch <= 0);
+    if (p->auto_shape) {
+        // The streaming kernels' shape: two steps per launch, tasks of as many rows
+        // as leave 16 warps per SM (a grid of a few hundred thousand cells is bound
+        // by the chain of row loads in a task, a large one by the rows a task
+        // computes twice).  301 x 151, one shot: 3.9 us per step with 1 row, 49 us
+        // with the 32-row, one-step tasks that used to be the default.
+        long long rows_all = 0;
+        for (int s = 0; s < nshots; ++s) rows_all += std::max(shots[s].nx, 0);
+        const long long strips = (g.nz + 59) / 60;
+        p->vec = 2;
+        p->tsteps = 2;
+        p->rows = 24;
+        while (p->rows > 1 && rows_all / p->rows * strips < 148 * 16) p->rows /= 2;
+        p->warps = 4;
+        p->prefetch = p->rows >= 12 ? 3 : 1;
     }
     const int W = 30 * p->vec;
     p->nstrips = (g.nz + W - 1) / W;
@@ -652,7 +950,7 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     p->n_rec_ptr = rec_ptr.size();
     p->n_src_ent = std::max<size_t>(src_ent.size(), 1);
     p->n_rec_ent = std::max<size_t>(rec_ent.size(), 1);
-    rc |= dalloc(&p->d_flags, nshots);
+    rc |= dalloc(&p->d_flags, (size_t)nshots + 1);  // the last word: the resident kernel's error
     rc |= dalloc(&p->d_fail_seq, nshots);
     rc |= dalloc(&p->d_sponge, std::max(g.absorbing_frame, 1));
     for (int b = 0; b < 2 && !rc; ++b)
@@ -692,9 +990,22 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
         delete p;
         return fail(RTM_E_CUDA, "plan upload failed: %s", cudaGetErrorString(e));
     }
+    if (p->auto_shape) {
+        p->src_ptr_h = std::move(src_ptr);
+        p->src_ent_h = std::move(src_ent);
+        p->rec_ptr_h = std::move(rec_ptr);
+        p->rec_ent_h = std::move(rec_ent);
+        if (int r2 = resident_setup(p, false)) {
+            plan_free(p);
+            delete p;
+            return r2;
+        }
+    }
     *out = p;
     return RTM_OK;
 }
+
+int rtm_plan_resident(const rtm_plan *p) { return p && p->res.r > 0 ? 1 : 0; }
 
 int rtm_plan_destroy(rtm_plan *p) {
     if (!p) return RTM_OK;
@@ -761,6 +1072,8 @@ int rtm_plan_set_model(rtm_plan *p, const float *mu, const float *lam, const flo
         p->d_mat[M_MYZ], surface ? p->d_surface : nullptr);
     CUDA_TRY(cudaGetLastError());
     p->has_surface = surface != nullptr;
+    if (p->auto_shape && p->has_surface != p->res.surface)
+        if (int rc = resident_setup(p, p->has_surface)) return rc;
     p->model_set = true;
     return RTM_OK;
 }
@@ -799,7 +1112,8 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
     if (save)
         for (float *b : {snap_u, snap_v, snap_w}) bs.add(b, rtm_plan_snapshot_floats(p, nsnap) * sizeof(float));
     if (int rc = bs.begin(s)) return rc;
-    if (int rc = zero_state(p, s)) return rc;
+    const bool resident = p->res.r > 0 && !p->cb;
+    if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
     // Snapshot slots the time loop never reaches ((k+1)*isnap > nt-1) stay
     // zero, like the reference's zero-initialised fields (fm:533-535).
     if (save)
@@ -838,7 +1152,7 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
     // a launch ends at each of them
     auto cb_at = [&](int it) { return p->cb && p->cb_every > 0 && it % p->cb_every == 0; };
     const std::vector<LoopLaunch> sched =
-        loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !cb_at(it); });
+        resident ? std::vector<LoopLaunch>() : loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !cb_at(it); });
     auto loop = [&](cudaStream_t ls) -> int {
         for (size_t L = 0; L < sched.size(); ++L) {
             const int it = sched[L].it;
@@ -868,12 +1182,31 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
     const std::vector<unsigned long long> key = {U(wavelets), U(snap_u), U(snap_v), U(snap_w),
                                                  (unsigned long long)save, (unsigned long long)isnap,
                                                  (unsigned long long)check_interval};
-    if (p->cb) {  // host callbacks in the loop: direct launches
+    if (resident) {
+        ResParams rp;
+        resident_params(p, rp, 0);
+        for (int c = 0; c < 3; ++c) {
+            rp.wav[c] = sp.wav[c];
+            rp.seis[c] = sp.seis[c];
+            rp.snap[c] = sp.snap[c];
+        }
+        rp.code_base = 1;
+        rp.nsnap = nsnap;
+        rp.it1 = nt;
+        rp.check_interval = check_interval;
+        if (nsnap > 0) {
+            rp.isnap = isnap;
+            rp.snap_base = rp.snap_lo = 1;
+            rp.snap_hi = nsnap;
+        }
+        if (int rc = resident_run(p, rp, 0, s)) return rc;
+        p->live = 0;
+    } else if (p->cb) {  // host callbacks in the loop: direct launches
         if (int rc = loop(s)) return rc;
     } else if (int rc = run_loop(p, p->g_fwd, key, s, loop)) {
         return rc;
     }
-    p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
+    if (!resident) p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
     p->launches += (long long)sched.size();
     if (seis && p->nrec_total) {
         if (int rc = transpose(p->d_seis_t, seis, 3, nt, p->nrec_total, s)) return rc;
@@ -884,10 +1217,8 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
             const int it = (k + 1) * isnap;
             isnaps_out[k] = it <= nt - 1 ? it : 0;  // fm:572; slots never reached stay 0
         }
-    if (flags) {
-        CUDA_TRY(cudaMemcpyAsync(flags, p->d_flags, p->nshots * sizeof(int), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(cudaStreamSynchronize(s));
-    }
+    if (flags)
+        if (int rc = read_status(p, flags, s)) return rc;
     if (int rc = bs.end(s)) return rc;
     return RTM_OK;
 }
@@ -919,7 +1250,11 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
     bs.add(image, (size_t)3 * p->g.nx * p->g.nz * sizeof(float));
     bs.add(stack, (size_t)3 * p->g.nx * p->g.nz * sizeof(double));
     if (int rc = bs.begin(s)) return rc;
-    if (int rc = zero_state(p, s)) return rc;
+    // the resident kernel images at every multiple of isnap that has a slot
+    bool resident = p->res.r > 0 && !p->cb;
+    for (int k = 0; k < num_snaps; ++k)
+        if ((long long)(k + 1) * isnap <= nt - 1 && isnaps[k] != (k + 1) * isnap) resident = false;
+    if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
     const size_t img_floats = (size_t)p->rows_total * p->pitch;
     for (int c = 0; c < 3; ++c)
         if (p->d_img[c]) {
@@ -955,7 +1290,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
     // (backward_modeling.py:565-569): a launch ends at each of them
     auto cb_at = [&](int it) { return p->cb && snap_of[it] >= 0; };
     const std::vector<LoopLaunch> sched =
-        loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !cb_at(it); });
+        resident ? std::vector<LoopLaunch>() : loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !cb_at(it); });
     auto loop = [&](cudaStream_t ls) -> int {
         for (size_t L = 0; L < sched.size(); ++L) {
             const int it = sched[L].it;
@@ -986,12 +1321,32 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
                                            (unsigned long long)isnap, (unsigned long long)check_interval};
     for (int it = 0; it < nt; ++it)
         if (snap_of[it] >= 0) key.push_back(((unsigned long long)it << 32) | (unsigned)snap_of[it]);
-    if (p->cb) {  // host callbacks in the loop: direct launches
+    if (resident) {
+        ResParams rp;
+        resident_params(p, rp, 1);
+        for (int c = 0; c < 3; ++c) {
+            rp.obs[c] = sp.obs[c];
+            rp.snap[c] = sp.snap[c];
+            rp.img[c] = sp.img[c];
+            rp.imgc[c] = sp.imgc[c];
+        }
+        rp.code_base = 4;
+        rp.nsnap = num_snaps;
+        rp.it1 = nt;
+        rp.check_interval = check_interval;
+        if (num_snaps > 0) {
+            rp.isnap = isnap;
+            rp.snap_base = rp.snap_lo = 1;
+            rp.snap_hi = num_snaps;
+        }
+        if (int rc = resident_run(p, rp, 1, s)) return rc;
+        p->live = 0;
+    } else if (p->cb) {  // host callbacks in the loop: direct launches
         if (int rc = loop(s)) return rc;
     } else if (int rc = run_loop(p, p->g_bwd, key, s, loop)) {
         return rc;
     }
-    p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
+    if (!resident) p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
     p->launches += (long long)sched.size();
     const int blocks = 148 * 8;
     const size_t n = (size_t)p->g.nx * p->g.nz;
@@ -1049,8 +1404,11 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
             ++p->launches;
         }
     }
-    if (flags) CUDA_TRY(cudaMemcpyAsync(flags, p->d_flags, p->nshots * sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (flags || norm) CUDA_TRY(cudaStreamSynchronize(s));  // scratch is freed on return
+    if (flags) {
+        if (int rc = read_status(p, flags, s)) return rc;
+    } else if (norm) {
+        CUDA_TRY(cudaStreamSynchronize(s));  // scratch is freed on return
+    }
     if (int rc = bs.end(s)) return rc;
     return RTM_OK;
 }

@@ -87,6 +87,11 @@ class Plan:
         n = int(_lib.lib().rtm_plan_snapshot_floats(self.h, int(nsnap)))
         return torch.empty(max(n, 1), dtype=torch.float32, device=self.device)
 
+    def resident(self):
+        """True when rtm_forward / rtm_backward keep the wavefield on the chip
+        (rtm_plan_resident)."""
+        return bool(_lib.lib().rtm_plan_resident(self.h))
+
     def launch_count(self):
         return int(_lib.lib().rtm_plan_launch_count(self.h))
 
