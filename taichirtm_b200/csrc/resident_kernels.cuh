@@ -29,46 +29,10 @@
 #include <cuda_runtime.h>
 #include <limits.h>
 
+#include "f32x2.cuh"
 #include "step_kernels.cuh"
 
 namespace rtm {
-
-// ---- packed FP32 pairs.  add / sub are the packed IEEE operations.  A product
-// is fma(a, b, -0.0) with the -0.0 opaque to the compiler (a kernel argument):
-// exactly the rounded product, sign of zero included, and unlike mul.f32x2 it
-// cannot be fused with a following addition (ptxas 12.9 does fuse those, even
-// with -fmad=false: 68,271 of 524,288 random chains f + (d b)(a + b) then
-// differ from the IEEE sequence; 0 with this form).
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2_pack(float lo, float hi) {
-    f2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float f2_lo(f2 a) {
-    return __uint_as_float((unsigned)a);
-}
-__device__ __forceinline__ float f2_hi(f2 a) {
-    return __uint_as_float((unsigned)(a >> 32));
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
-    f2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b, f2 neg_zero) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(neg_zero));
-    return d;
-}
-__device__ __forceinline__ f2 f2_sel(bool lo, bool hi, f2 a, f2 b) {
-    return f2_pack(lo ? f2_lo(a) : f2_lo(b), hi ? f2_hi(a) : f2_hi(b));
-}
 
 constexpr int RES_COLS = 64;             // tile columns: 32 lanes x 2
 constexpr int RES_HALO = 4;              // H: halo rows / columns, steps per exchange

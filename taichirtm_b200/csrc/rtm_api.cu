@@ -335,11 +335,11 @@ cudaError_t launch_step2(const StepParams &sp, int warps, cudaStream_t s) {
     size_t smem = 0;
     if constexpr (RING) {
         constexpr size_t kMaxSmem = 227 * 1024;  // per-block opt-in limit
-        smem = (size_t)warps * ring2_smem_per_warp<MODE, VEC>();
+        smem = (size_t)warps * ring2_smem_per_warp<MODE, VEC>(sp.surface != nullptr);
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
         static bool attr_set = false;  // per instantiation; raises the 48 KB default
         if (!attr_set) {
-            const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<MODE, VEC>(), kMaxSmem);
+            const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<MODE, VEC>(true), kMaxSmem);
             cudaError_t e = cudaFuncSetAttribute(step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
             if (e != cudaSuccess) return e;
@@ -478,6 +478,7 @@ void fill_common(const rtm_plan *p, StepParams &sp) {
     sp.inv_dx = (float)(1.0 / p->g.dx);
     sp.inv_dz = (float)(1.0 / p->g.dz);
     sp.src_factor = (float)(dt * p->g.dx * p->g.dz);  // forward_modeling.py:430
+    sp.neg_zero = -0.0f;
     sp.sponge = p->d_sponge;
     sp.work = p->d_work;
     sp.n_work = p->n_work;

@@ -36,27 +36,60 @@
 #pragma once
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "step_kernels.cuh"
 
 namespace rtm {
 
+// A lane's VEC columns of one row, as VEC / 2 packed pairs (f32x2.cuh).
 template <int VEC>
-struct SigRow { float xx[VEC], zz[VEC], xz[VEC], yx[VEC], yz[VEC]; };
+struct SigRow { f2 xx[VEC / 2], zz[VEC / 2], xz[VEC / 2], yx[VEC / 2], yz[VEC / 2]; };
 template <int VEC>
-struct VelRow { float u[VEC], w[VEC], v[VEC]; };
+struct VelRow { f2 u[VEC / 2], w[VEC / 2], v[VEC / 2]; };
 template <int VEC>
-struct MatRow { float lam[VEC], mu[VEC], mxz[VEC], myx[VEC], myz[VEC], sm[VEC]; };
+struct MatRow { f2 lam[VEC / 2], mu[VEC / 2], mxz[VEC / 2], myx[VEC / 2], myz[VEC / 2], sm[VEC / 2]; };
 
-template <int VEC>
-__device__ __forceinline__ void zero_arr(float (&a)[VEC]) {
+template <int N>
+__device__ __forceinline__ void zero_arr(f2 (&a)[N]) {
 #pragma unroll
-    for (int q = 0; q < VEC; ++q) a[q] = 0.f;
+    for (int q = 0; q < N; ++q) a[q] = 0ull;
 }
 
-template <int VEC>
-__device__ __forceinline__ void copy_arr(float (&d)[VEC], const float (&s)[VEC]) {
+template <int N>
+__device__ __forceinline__ void copy_arr(f2 (&d)[N], const f2 (&s)[N]) {
 #pragma unroll
-    for (int q = 0; q < VEC; ++q) d[q] = s[q];
+    for (int q = 0; q < N; ++q) d[q] = s[q];
+}
+
+// Vector loads and stores of VEC / 2 pairs.
+template <int N>
+__device__ __forceinline__ void ldp(f2 (&v)[N], const float *__restrict__ p) {
+    if constexpr (N == 2) {
+        const ulonglong2 t = ldg_chk(reinterpret_cast<const ulonglong2 *>(p));
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        v[0] = ldg_chk(reinterpret_cast<const f2 *>(p));
+    }
+}
+template <int N>
+__device__ __forceinline__ void stp(float *__restrict__ p, const f2 (&v)[N]) {
+    if (!RTM_DBG_OK(p, N * sizeof(f2))) return;
+    if constexpr (N == 2) *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v[0], v[1]);
+    else *reinterpret_cast<f2 *>(p) = v[0];
+}
+template <int N>
+__device__ __forceinline__ void unpack(float (&d)[2 * N], const f2 (&s)[N]) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) { d[2 * q] = f2_lo(s[q]); d[2 * q + 1] = f2_hi(s[q]); }
+}
+// Differences with the next lower / higher column; nb: the neighbouring lane's.
+template <int N>
+__device__ __forceinline__ f2 diff_lo(const f2 (&x)[N], int q, float nb) {
+    return f2_pack(f2_lo(x[q]) - (q > 0 ? f2_hi(x[q > 0 ? q - 1 : 0]) : nb), f2_hi(x[q]) - f2_lo(x[q]));
+}
+template <int N>
+__device__ __forceinline__ f2 diff_hi(const f2 (&x)[N], int q, float nb) {
+    return f2_pack(f2_hi(x[q]) - f2_lo(x[q]), (q < N - 1 ? f2_lo(x[q < N - 1 ? q + 1 : 0]) : nb) - f2_hi(x[q]));
 }
 
 // Plain (coherent) vector load for the Kahan image: one thread may read a
@@ -89,10 +122,11 @@ __device__ __forceinline__ void ldv_coherent(float (&v)[VEC], float *p) {
 // 1/rho_u, 1/rho_w; SH myx, myz, 1/rho; the surface mask.
 constexpr int RING2_ROWS = 4;
 template <int MODE>
-__host__ __device__ constexpr int ring2_fields() { return ((MODE & 1) ? 5 : 0) + ((MODE & 2) ? 3 : 0) + 1; }
+__host__ __device__ constexpr int ring2_fields() { return ((MODE & 1) ? 5 : 0) + ((MODE & 2) ? 3 : 0); }
+constexpr int RING2_STATE_ROWS = 3;
 template <int MODE, int VEC>
-__host__ __device__ constexpr size_t ring2_smem_per_warp() {
-    return (size_t)RING2_ROWS * ring2_fields<MODE>() * 32 * VEC * sizeof(float);
+__host__ __device__ constexpr size_t ring2_smem_per_warp(bool surface) {
+    return ((size_t)RING2_ROWS * (ring2_fields<MODE>() + (surface ? 1 : 0)) + RING2_STATE_ROWS * ring2_fields<MODE>()) * 32 * VEC * sizeof(float);
 }
 
 // STOREA: also store step A's state (rows [ia, ib), into p.souta), for the
@@ -138,13 +172,14 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     // factored into a column part fixed for the task (here, once per lane)
     // and a warp-uniform row part (ColRow below): the same cells are interior
     // and the same sponge entry is chosen as by interior() and sponge_coef().
-    bool col_in[VEC], col_sp[VEC];
+    bool col_sp[VEC];
+    unsigned col_m[VEC];  // all ones for an interior column
     int col_db[VEC];
     float col_cr[VEC];
 #pragma unroll
     for (int q = 0; q < VEC; ++q) {
         const int j = c0 + q;
-        col_in[q] = (unsigned)(j - 1) < (unsigned)(nz - 2);
+        col_m[q] = (unsigned)(j - 1) < (unsigned)(nz - 2) ? ~0u : 0u;
         col_db[q] = nz - 1 - j;  // distance to the bottom edge
         col_sp[q] = col_db[q] >= 0 && col_db[q] < p.fw;
         col_cr[q] = col_sp[q] ? ldg_chk(p.sponge + col_db[q]) : 1.0f;
@@ -152,15 +187,16 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     const long long soff = sh.state_off + (long long)(c0 + COL_OFF);
     const long long moff = (long long)sh.x0 * P + (long long)(c0 + COL_OFF);
     const float dt = p.dt, idx = p.inv_dx, idz = p.inv_dz;
-    const float sdt = DIR == 0 ? dt : -dt;
+    const f2 dt2 = f2_pack(dt, dt), idx2 = f2_pack(idx, idx), idz2 = f2_pack(idz, idz), nz2 = f2_pack(p.neg_zero, p.neg_zero);
+    constexpr int NP = VEC / 2;
     // CKPT: scale block of row -1 of this task's strip (padded row 0 of the shot)
     long long ck_blk0 = 0;
     if constexpr (CKPT) ck_blk0 = (sh.state_off / P) * p.ck.nblk + (wk.y & 0xFFFFF) * (W / ckpt_block_cols(VEC));
     // rows -1 and nx are the zero pad rows of the shot block (and of the
     // material window); rows beyond them read the pad row (header comment)
     auto rowc = [&](int i) { return min(max(i, -1), nx); };
-    auto LSt = [&](float (&v)[VEC], int f, int i) { ldv<VEC>(v, p.sin[f] + soff + (long long)(rowc(i) + 1) * P); };
-    auto LMt = [&](float (&v)[VEC], int m, int i) { ldv<VEC>(v, p.mat[m] + moff + (long long)(rowc(i) + 1) * P); };
+    auto LSt = [&](f2 (&v)[NP], int f, int i) { ldp<NP>(v, p.sin[f] + soff + (long long)(rowc(i) + 1) * P); };
+    auto LMt = [&](f2 (&v)[NP], int m, int i) { ldp<NP>(v, p.mat[m] + moff + (long long)(rowc(i) + 1) * P); };
     auto load_sig = [&](int i, Sig &s) {
         if constexpr (PSV) { LSt(s.xx, F_SXX, i); LSt(s.zz, F_SZZ, i); LSt(s.xz, F_SXZ, i); }
         if constexpr (SH) { LSt(s.yx, F_SYX, i); LSt(s.yz, F_SYZ, i); }
@@ -177,23 +213,57 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
         if constexpr (PSV) { LMt(m.lam, M_LAM, i); LMt(m.mu, M_MU, i); LMt(m.mxz, M_MXZ, i); }
         if constexpr (SH) { LMt(m.myx, M_MYX, i); LMt(m.myz, M_MYZ, i); }
         if (p.surface) {
-            ldv<VEC>(m.sm, p.surface + moff + (long long)(rowc(i) + 1) * P);
+            ldp<NP>(m.sm, p.surface + moff + (long long)(rowc(i) + 1) * P);
         } else {
 #pragma unroll
-            for (int q = 0; q < VEC; ++q) m.sm[q] = 1.f;
+            for (int q = 0; q < NP; ++q) m.sm[q] = f2_pack(1.f, 1.f);
         }
     };
     // ---- material ring (RING): slot of a row, copy-in, read-back
     constexpr int NRF = ring2_fields<MODE>();
     constexpr int RF_LAM = 0, RF_MU = 1, RF_MXZ = 2, RF_IRU = 3, RF_IRW = 4;
     constexpr int RF_MYX = PSV ? 5 : 0, RF_MYZ = RF_MYX + 1, RF_IR = RF_MYX + 2;
-    constexpr int RF_SM = NRF - 1;
+    constexpr int RF_SM = NRF;
+    const int nrf = NRF + (p.surface ? 1 : 0);  // the surface mask's rows only where there is one
     extern __shared__ float step2_smem[];
     static_assert((RING2_ROWS & (RING2_ROWS - 1)) == 0, "the ring slot is the row modulo a power of two");
     // this lane's VEC floats of slot 0, field 0; a (slot, field) is a fixed
     // 32-bit offset from it (rows >= -2: row & (RING2_ROWS - 1) is the slot)
-    float *const ring = step2_smem + (UNI ? 0 : (int)(threadIdx.x >> 5) * (RING2_ROWS * NRF * 32 * VEC)) + lane * VEC;
-    auto rslot = [&](int row, int f) { return ring + ((row & (RING2_ROWS - 1)) * NRF + f) * (32 * VEC); };
+    float *const ring = step2_smem + (UNI ? 0 : (int)(threadIdx.x >> 5) * ((RING2_ROWS * nrf + RING2_STATE_ROWS * NRF) * 32 * VEC)) + lane * VEC;
+    float *const sring = ring + RING2_ROWS * nrf * (32 * VEC);
+    auto rslot = [&](int row, int f) { return ring + ((row & (RING2_ROWS - 1)) * nrf + f) * (32 * VEC); };
+    // state ring: slot 0, 1, 2 of the rows in turn; fields as NFIELD of the modes
+    auto sslot = [&](int slot, int f) { return sring + (slot * NRF + f) * (32 * VEC); };
+    // stress of row `row` and velocity of row `vrow` into a slot
+    auto state_issue = [&](int slot, int row, int vrow) {
+        if (row <= ib + 1) {
+            auto put = [&](int f, int field, int r) {
+                cp_async_vec<VEC>(sslot(slot, f), p.sin[field] + soff + (long long)(rowc(r) + 1) * P);
+            };
+            constexpr int o = PSV ? 5 : 0;
+            if constexpr (PSV) {
+                put(0, F_SXX, row); put(1, F_SZZ, row); put(2, F_SXZ, row);
+                put(3, F_U, vrow); put(4, F_W, vrow);
+            }
+            if constexpr (SH) { put(o, F_SYX, row); put(o + 1, F_SYZ, row); put(o + 2, F_V, vrow); }
+        }
+        cp_async_commit();
+    };
+    auto rd_state = [&](int slot, Sig &sg, Vel &v) {
+        auto get = [&](int f, f2 (&x)[NP]) {
+            const float *a = sslot(slot, f);
+            if constexpr (NP == 2) {
+                const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(a);
+                x[0] = t.x; x[1] = t.y;
+            } else {
+                x[0] = *reinterpret_cast<const f2 *>(a);
+            }
+        };
+        constexpr int o = PSV ? 5 : 0;
+        if constexpr (PSV) { get(0, sg.xx); get(1, sg.zz); get(2, sg.xz); get(3, v.u); get(4, v.w); }
+        if constexpr (SH) { get(o, sg.yx); get(o + 1, sg.yz); get(o + 2, v.v); }
+    };
+    (void)state_issue; (void)rd_state;
     auto ring_issue = [&](int row) {
         auto put = [&](int f, const float *src) {
             cp_async_vec<VEC>(rslot(row, f), src + moff + (long long)(rowc(row) + 1) * P);
@@ -206,10 +276,14 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
         if (p.surface) put(RF_SM, p.surface);
         cp_async_commit();  // one group per issued row, so the group counts stay aligned
     };
-    auto rd_ring = [&](int row, int f, float (&v)[VEC]) {
+    auto rd_ring = [&](int row, int f, f2 (&v)[NP]) {
         const float *s = rslot(row, f);
-#pragma unroll
-        for (int q = 0; q < VEC; ++q) v[q] = s[q];
+        if constexpr (NP == 2) {
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(s);
+            v[0] = t.x; v[1] = t.y;
+        } else {
+            v[0] = *reinterpret_cast<const f2 *>(s);
+        }
     };
     auto ring_ir = [&](int row, Vel &v) {
         if constexpr (PSV) { rd_ring(row, RF_IRU, v.u); rd_ring(row, RF_IRW, v.w); }
@@ -222,89 +296,72 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             rd_ring(row, RF_SM, m.sm);
         } else {
 #pragma unroll
-            for (int q = 0; q < VEC; ++q) m.sm[q] = 1.f;
+            for (int q = 0; q < NP; ++q) m.sm[q] = f2_pack(1.f, 1.f);
         }
     };
     (void)ring_issue; (void)ring_ir; (void)ring_mat;
 
     auto cp_sig = [&](Sig &d, const Sig &s) {
-        if constexpr (PSV) { copy_arr<VEC>(d.xx, s.xx); copy_arr<VEC>(d.zz, s.zz); copy_arr<VEC>(d.xz, s.xz); }
-        if constexpr (SH) { copy_arr<VEC>(d.yx, s.yx); copy_arr<VEC>(d.yz, s.yz); }
+        if constexpr (PSV) { copy_arr<NP>(d.xx, s.xx); copy_arr<NP>(d.zz, s.zz); copy_arr<NP>(d.xz, s.xz); }
+        if constexpr (SH) { copy_arr<NP>(d.yx, s.yx); copy_arr<NP>(d.yz, s.yz); }
     };
     auto cp_vel = [&](Vel &d, const Vel &s) {
-        if constexpr (PSV) { copy_arr<VEC>(d.u, s.u); copy_arr<VEC>(d.w, s.w); }
-        if constexpr (SH) copy_arr<VEC>(d.v, s.v);
+        if constexpr (PSV) { copy_arr<NP>(d.u, s.u); copy_arr<NP>(d.w, s.w); }
+        if constexpr (SH) copy_arr<NP>(d.v, s.v);
     };
     auto cp_mat = [&](Mat &d, const Mat &s) {
-        if constexpr (PSV) { copy_arr<VEC>(d.lam, s.lam); copy_arr<VEC>(d.mu, s.mu); copy_arr<VEC>(d.mxz, s.mxz); }
-        if constexpr (SH) { copy_arr<VEC>(d.myx, s.myx); copy_arr<VEC>(d.myz, s.myz); }
-        copy_arr<VEC>(d.sm, s.sm);
+        if constexpr (PSV) { copy_arr<NP>(d.lam, s.lam); copy_arr<NP>(d.mu, s.mu); copy_arr<NP>(d.mxz, s.mxz); }
+        if constexpr (SH) { copy_arr<NP>(d.myx, s.myx); copy_arr<NP>(d.myz, s.myz); }
+        copy_arr<NP>(d.sm, s.sm);
     };
     auto zero_sig = [&](Sig &s) {
-        if constexpr (PSV) { zero_arr<VEC>(s.xx); zero_arr<VEC>(s.zz); zero_arr<VEC>(s.xz); }
-        if constexpr (SH) { zero_arr<VEC>(s.yx); zero_arr<VEC>(s.yz); }
+        if constexpr (PSV) { zero_arr<NP>(s.xx); zero_arr<NP>(s.zz); zero_arr<NP>(s.xz); }
+        if constexpr (SH) { zero_arr<NP>(s.yx); zero_arr<NP>(s.yz); }
     };
     auto zero_vel = [&](Vel &v) {
-        if constexpr (PSV) { zero_arr<VEC>(v.u); zero_arr<VEC>(v.w); }
-        if constexpr (SH) zero_arr<VEC>(v.v);
+        if constexpr (PSV) { zero_arr<NP>(v.u); zero_arr<NP>(v.w); }
+        if constexpr (SH) zero_arr<NP>(v.v);
     };
 
     // Velocity update of row r (step time t), the arithmetic of step_kernel.
     // Forward: sc = stress row r, sp = row r-1.  Backward: sc = row r+1,
     // sp = row r.  vo = velocity of row r before the update.  FAST (every
     // column of the lane interior) drops the interior select, nothing else.
+    // Edge cells keep their value: their increment is cleared bitwise, so not
+    // even a NaN of a failing shot gets in.
+    auto clip = [&](f2 d, int q, unsigned rm) -> f2 {
+        return (f2)((unsigned)(d >> 32) & col_m[2 * q + 1] & rm) << 32 | ((unsigned)d & col_m[2 * q] & rm);
+    };
     auto vel_cells = [&](auto fast_tag, int r, const Sig &sc, const Sig &sp, const Vel &vo, const Vel &ir,
                          Vel &out, float zz_nb, float xz_nb, float yz_nb) {
         constexpr bool FAST = decltype(fast_tag)::value;
-        const bool row_in = (unsigned)(r - 1) < (unsigned)(nx - 2);
+        unsigned rm = ~0u;
+        if constexpr (!FAST) rm = (unsigned)(r - 1) < (unsigned)(nx - 2) ? ~0u : 0u;
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-            bool in = true;
-            if constexpr (!FAST) in = row_in && col_in[q];
+        for (int q = 0; q < NP; ++q) {
             if constexpr (PSV) {
-                float du, dw;
-                if constexpr (DIR == 0) {
-                    const float sxz_jm = q > 0 ? sc.xz[q - 1] : xz_nb;
-                    const float szz_jm = q > 0 ? sc.zz[q - 1] : zz_nb;
-                    const float sxx_x = (sc.xx[q] - sp.xx[q]) * idx;  // fm:332
-                    const float szz_z = (sc.zz[q] - szz_jm) * idz;    // fm:333
-                    const float sxz_x = (sc.xz[q] - sp.xz[q]) * idx;  // fm:334
-                    const float sxz_z = (sc.xz[q] - sxz_jm) * idz;    // fm:335
-                    du = (sxx_x + sxz_z) * dt * ir.u[q];              // fm:339
-                    dw = (sxz_x + szz_z) * dt * ir.w[q];              // fm:340
-                } else {
-                    const float sxz_jp = q < VEC - 1 ? sp.xz[q + 1] : xz_nb;
-                    const float szz_jp = q < VEC - 1 ? sp.zz[q + 1] : zz_nb;
-                    const float sxx_x = (sc.xx[q] - sp.xx[q]) * idx;  // bm:333
-                    const float szz_z = (szz_jp - sp.zz[q]) * idz;    // bm:334
-                    const float sxz_x = (sc.xz[q] - sp.xz[q]) * idx;  // bm:335
-                    const float sxz_z = (sxz_jp - sp.xz[q]) * idz;    // bm:336
-                    du = -(sxx_x + sxz_z) * dt * ir.u[q];             // bm:340
-                    dw = -(sxz_x + szz_z) * dt * ir.w[q];             // bm:341
-                }
-                if constexpr (FAST) {
-                    out.u[q] = vo.u[q] + du;
-                    out.w[q] = vo.w[q] + dw;
-                } else {
-                    out.u[q] = in ? vo.u[q] + du : vo.u[q];
-                    out.w[q] = in ? vo.w[q] + dw : vo.w[q];
-                }
+                const f2 sxx_x = f2_mul(f2_sub(sc.xx[q], sp.xx[q]), idx2, nz2);  // fm:332, bm:333
+                const f2 sxz_x = f2_mul(f2_sub(sc.xz[q], sp.xz[q]), idx2, nz2);  // fm:334, bm:335
+                f2 dzz, dxz;
+                if constexpr (DIR == 0) { dzz = diff_lo(sc.zz, q, zz_nb); dxz = diff_lo(sc.xz, q, xz_nb); }
+                else { dzz = diff_hi(sp.zz, q, zz_nb); dxz = diff_hi(sp.xz, q, xz_nb); }
+                const f2 szz_z = f2_mul(dzz, idz2, nz2);                          // fm:333, bm:334
+                const f2 sxz_z = f2_mul(dxz, idz2, nz2);                          // fm:335, bm:336
+                f2 du = f2_mul(f2_mul(f2_add(sxx_x, sxz_z), dt2, nz2), ir.u[q], nz2);  // fm:339, bm:340 (negated)
+                f2 dw = f2_mul(f2_mul(f2_add(sxz_x, szz_z), dt2, nz2), ir.w[q], nz2);  // fm:340, bm:341
+                if constexpr (!FAST) { du = clip(du, q, rm); dw = clip(dw, q, rm); }
+                out.u[q] = DIR == 0 ? f2_add(vo.u[q], du) : f2_sub(vo.u[q], du);
+                out.w[q] = DIR == 0 ? f2_add(vo.w[q], dw) : f2_sub(vo.w[q], dw);
             }
             if constexpr (SH) {
-                float dv;
-                if constexpr (DIR == 0) {
-                    const float syz_jm = q > 0 ? sc.yz[q - 1] : yz_nb;
-                    const float syx_x = (sc.yx[q] - sp.yx[q]) * idx;  // fm:343
-                    const float syz_z = (sc.yz[q] - syz_jm) * idz;    // fm:344
-                    dv = (syx_x + syz_z) * dt * ir.v[q];              // fm:347
-                } else {
-                    const float syz_jp = q < VEC - 1 ? sp.yz[q + 1] : yz_nb;
-                    const float syx_x = (sc.yx[q] - sp.yx[q]) * idx;  // bm:343
-                    const float syz_z = (syz_jp - sp.yz[q]) * idz;    // bm:344
-                    dv = -(syx_x + syz_z) * dt * ir.v[q];             // bm:345
-                }
-                if constexpr (FAST) out.v[q] = vo.v[q] + dv;
-                else out.v[q] = in ? vo.v[q] + dv : vo.v[q];
+                const f2 syx_x = f2_mul(f2_sub(sc.yx[q], sp.yx[q]), idx2, nz2);  // fm:343, bm:343
+                f2 dyz;
+                if constexpr (DIR == 0) dyz = diff_lo(sc.yz, q, yz_nb);
+                else dyz = diff_hi(sp.yz, q, yz_nb);
+                const f2 syz_z = f2_mul(dyz, idz2, nz2);                          // fm:344, bm:344
+                f2 dv = f2_mul(f2_mul(f2_add(syx_x, syz_z), dt2, nz2), ir.v[q], nz2);  // fm:347, bm:345
+                if constexpr (!FAST) dv = clip(dv, q, rm);
+                out.v[q] = DIR == 0 ? f2_add(vo.v[q], dv) : f2_sub(vo.v[q], dv);
             }
         }
     };
@@ -313,16 +370,16 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
         float zz_nb = 0.f, xz_nb = 0.f, yz_nb = 0.f;
         if constexpr (DIR == 0) {
             if constexpr (PSV) {
-                zz_nb = __shfl_up_sync(FULL, sc.zz[VEC - 1], 1);
-                xz_nb = __shfl_up_sync(FULL, sc.xz[VEC - 1], 1);
+                zz_nb = __shfl_up_sync(FULL, f2_hi(sc.zz[NP - 1]), 1);
+                xz_nb = __shfl_up_sync(FULL, f2_hi(sc.xz[NP - 1]), 1);
             }
-            if constexpr (SH) yz_nb = __shfl_up_sync(FULL, sc.yz[VEC - 1], 1);
+            if constexpr (SH) yz_nb = __shfl_up_sync(FULL, f2_hi(sc.yz[NP - 1]), 1);
         } else {
             if constexpr (PSV) {
-                zz_nb = __shfl_down_sync(FULL, sp.zz[0], 1);
-                xz_nb = __shfl_down_sync(FULL, sp.xz[0], 1);
+                zz_nb = __shfl_down_sync(FULL, f2_lo(sp.zz[0]), 1);
+                xz_nb = __shfl_down_sync(FULL, f2_lo(sp.xz[0]), 1);
             }
-            if constexpr (SH) yz_nb = __shfl_down_sync(FULL, sp.yz[0], 1);
+            if constexpr (SH) yz_nb = __shfl_down_sync(FULL, f2_lo(sp.yz[0]), 1);
         }
         if (all_in(r)) vel_cells(std::true_type{}, r, sc, sp, vo, ir, out, zz_nb, xz_nb, yz_nb);
         else vel_cells(std::false_type{}, r, sc, sp, vo, ir, out, zz_nb, xz_nb, yz_nb);
@@ -339,15 +396,17 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                 const bool in = interior(r, en.x, nx, nz);
                 const float f = p.src_factor;
                 const size_t ti = (size_t)en.y * p.nt + t;
+                auto add = [&](f2 (&x)[NP], const f2 (&ir2)[NP], const float *wav, bool masked) {
+                    const float wf = ldg_chk(wav + ti) * f;
 #pragma unroll
-                for (int qq = 0; qq < VEC; ++qq) {
-                    if (qq != q) continue;
-                    if constexpr (PSV) {
-                        out.u[qq] += ldg_chk(p.wav[0] + ti) * f * (in ? ir.u[qq] : __int_as_float(0x7f800000));
-                        out.w[qq] += ldg_chk(p.wav[2] + ti) * f * (in ? ir.w[qq] : __int_as_float(0x7f800000));
+                    for (int k = 0; k < NP; ++k) {  // x + -0.0 is x: the other columns take part
+                        const float b = q & 1 ? f2_hi(ir2[k]) : f2_lo(ir2[k]);
+                        const float a = wf * (in || !masked ? b : __int_as_float(0x7f800000));
+                        x[k] = f2_add(x[k], f2_pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
                     }
-                    if constexpr (SH) out.v[qq] += ldg_chk(p.wav[1] + ti) * f * ir.v[qq];
-                }
+                };
+                if constexpr (PSV) { add(out.u, ir.u, p.wav[0], true); add(out.w, ir.w, p.wav[2], true); }
+                if constexpr (SH) add(out.v, ir.v, p.wav[1], false);
             }
         } else {
             if (no_rec) return;
@@ -357,15 +416,14 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                 const int q = en.x - c0;
                 if (q < 0 || q >= VEC) continue;
                 const size_t ti = (size_t)t * p.nrec_total + en.y;
+                auto add = [&](f2 (&x)[NP], const float *obs) {
+                    const float a = ldg_chk(obs + ti);
 #pragma unroll
-                for (int qq = 0; qq < VEC; ++qq) {
-                    if (qq != q) continue;
-                    if constexpr (PSV) {
-                        out.u[qq] += ldg_chk(p.obs[0] + ti);
-                        out.w[qq] += ldg_chk(p.obs[2] + ti);
-                    }
-                    if constexpr (SH) out.v[qq] += ldg_chk(p.obs[1] + ti);
-                }
+                    for (int k = 0; k < NP; ++k)
+                        x[k] = f2_add(x[k], f2_pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
+                };
+                if constexpr (PSV) { add(out.u, p.obs[0]); add(out.w, p.obs[2]); }
+                if constexpr (SH) add(out.v, p.obs[1]);
             }
         }
     };
@@ -383,83 +441,79 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
         // the left sponge and the cell is farther from the bottom, d = nx-1-r
         // likewise for the right sponge, d = the bottom distance if that is
         // in the sponge and no larger than both row distances (last wins)
-        bool row_in = true, ra = false, rb = false;
+        bool ra = false, rb = false;
+        unsigned rm = ~0u;
         int dr = 0;
         float cr_i = 1.0f, cr_dr = 1.0f;
         if constexpr (!FAST) {
-            row_in = (unsigned)(r - 1) < (unsigned)(nx - 2);
+            rm = (unsigned)(r - 1) < (unsigned)(nx - 2) ? ~0u : 0u;
             dr = nx - 1 - r;
             ra = r >= 0 && r < p.fw;
             rb = dr >= 0 && dr < p.fw;
             if (ra) cr_i = ldg_chk(p.sponge + r);
             if (rb) cr_dr = ldg_chk(p.sponge + dr);
         }
+        const f2 sdt2 = DIR == 0 ? dt2 : f2_pack(-dt, -dt);
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-            bool in = true;
-            float cr = 1.0f;
+        for (int q = 0; q < NP; ++q) {
+            f2 c = 0ull;
             if constexpr (!FAST) {
-                in = row_in && col_in[q];
-                if (ra && col_db[q] > r) cr = cr_i;
-                if (rb && col_db[q] > dr) cr = cr_dr;
-                if (col_sp[q] && r >= col_db[q] && dr >= col_db[q]) cr = col_cr[q];
+                float cr[2] = {1.0f, 1.0f};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = 2 * q + h;
+                    if (ra && col_db[k] > r) cr[h] = cr_i;
+                    if (rb && col_db[k] > dr) cr[h] = cr_dr;
+                    if (col_sp[k] && r >= col_db[k] && dr >= col_db[k]) cr[h] = col_cr[k];
+                }
+                c = f2_pack(cr[0], cr[1]);
             }
             if constexpr (PSV) {
-                float u_x, u_z, w_x, w_z;
+                f2 dux, dwx, duz, dwz;
                 if constexpr (DIR == 0) {
-                    const float uj = q < VEC - 1 ? va.u[q + 1] : nu;
-                    const float wj = q < VEC - 1 ? va.w[q + 1] : nw;
-                    u_x = (vb.u[q] - va.u[q]) * idx;   // fm:369
-                    u_z = (uj - va.u[q]) * idz;        // fm:370
-                    w_x = (vb.w[q] - va.w[q]) * idx;   // fm:371
-                    w_z = (wj - va.w[q]) * idz;        // fm:372
+                    dux = f2_sub(vb.u[q], va.u[q]); dwx = f2_sub(vb.w[q], va.w[q]);
+                    duz = diff_hi(va.u, q, nu); dwz = diff_hi(va.w, q, nw);
                 } else {
-                    const float uj = q > 0 ? va.u[q - 1] : nu;
-                    const float wj = q > 0 ? va.w[q - 1] : nw;
-                    u_x = (va.u[q] - vb.u[q]) * idx;   // bm:366
-                    u_z = (va.u[q] - uj) * idz;        // bm:367
-                    w_x = (va.w[q] - vb.w[q]) * idx;   // bm:368
-                    w_z = (va.w[q] - wj) * idz;        // bm:369
+                    dux = f2_sub(va.u[q], vb.u[q]); dwx = f2_sub(va.w[q], vb.w[q]);
+                    duz = diff_lo(va.u, q, nu); dwz = diff_lo(va.w, q, nw);
                 }
-                const float div = u_x + w_z;
-                const float sxx = base.xx[q] + sdt * (m.lam[q] * div + 2.0f * m.mu[q] * u_x);
-                const float szz = base.zz[q] + sdt * (m.lam[q] * div + 2.0f * m.mu[q] * w_z);
-                const float sxz = base.xz[q] + sdt * m.mxz[q] * (u_z + w_x);
+                const f2 u_x = f2_mul(dux, idx2, nz2), u_z = f2_mul(duz, idz2, nz2);  // fm:369-370, bm:366-367
+                const f2 w_x = f2_mul(dwx, idx2, nz2), w_z = f2_mul(dwz, idz2, nz2);  // fm:371-372, bm:368-369
+                const f2 ld = f2_mul(m.lam[q], f2_add(u_x, w_z), nz2), mu2 = f2_add(m.mu[q], m.mu[q]);
+                f2 dxx = f2_mul(sdt2, f2_add(ld, f2_mul(mu2, u_x, nz2)), nz2);
+                f2 dzz = f2_mul(sdt2, f2_add(ld, f2_mul(mu2, w_z, nz2)), nz2);
+                f2 dxz = f2_mul(f2_mul(sdt2, m.mxz[q], nz2), f2_add(u_z, w_x), nz2);
                 if constexpr (FAST) {
-                    os.xx[q] = sxx;
-                    os.zz[q] = szz;
-                    os.xz[q] = sxz;
+                    os.xx[q] = f2_add(base.xx[q], dxx);
+                    os.zz[q] = f2_add(base.zz[q], dzz);
+                    os.xz[q] = f2_add(base.xz[q], dxz);
                     ov.u[q] = va.u[q];
                     ov.w[q] = va.w[q];
                 } else {
-                    os.xx[q] = cr * (in ? sxx : base.xx[q]);
-                    os.zz[q] = (cr * (in ? szz : base.zz[q])) * m.sm[q];
-                    os.xz[q] = (cr * (in ? sxz : base.xz[q])) * m.sm[q];
-                    ov.u[q] = cr * va.u[q];
-                    ov.w[q] = cr * va.w[q];
+                    dxx = clip(dxx, q, rm); dzz = clip(dzz, q, rm); dxz = clip(dxz, q, rm);
+                    os.xx[q] = f2_mul(c, f2_add(base.xx[q], dxx), nz2);
+                    os.zz[q] = f2_mul(f2_mul(c, f2_add(base.zz[q], dzz), nz2), m.sm[q], nz2);
+                    os.xz[q] = f2_mul(f2_mul(c, f2_add(base.xz[q], dxz), nz2), m.sm[q], nz2);
+                    ov.u[q] = f2_mul(c, va.u[q], nz2);
+                    ov.w[q] = f2_mul(c, va.w[q], nz2);
                 }
             }
             if constexpr (SH) {
-                float v_x, v_z;
-                if constexpr (DIR == 0) {
-                    const float vj = q < VEC - 1 ? va.v[q + 1] : nv;
-                    v_x = (vb.v[q] - va.v[q]) * idx;   // fm:381
-                    v_z = (vj - va.v[q]) * idz;        // fm:382
-                } else {
-                    const float vj = q > 0 ? va.v[q - 1] : nv;
-                    v_x = (va.v[q] - vb.v[q]) * idx;   // bm:377
-                    v_z = (va.v[q] - vj) * idz;        // bm:378
-                }
-                const float syx = base.yx[q] + sdt * m.myx[q] * v_x;
-                const float syz = base.yz[q] + sdt * m.myz[q] * v_z;
+                f2 dvx, dvz;
+                if constexpr (DIR == 0) { dvx = f2_sub(vb.v[q], va.v[q]); dvz = diff_hi(va.v, q, nv); }
+                else { dvx = f2_sub(va.v[q], vb.v[q]); dvz = diff_lo(va.v, q, nv); }
+                const f2 v_x = f2_mul(dvx, idx2, nz2), v_z = f2_mul(dvz, idz2, nz2);  // fm:381-382, bm:377-378
+                f2 dyx = f2_mul(f2_mul(sdt2, m.myx[q], nz2), v_x, nz2);
+                f2 dyz = f2_mul(f2_mul(sdt2, m.myz[q], nz2), v_z, nz2);
                 if constexpr (FAST) {
-                    os.yx[q] = syx;
-                    os.yz[q] = syz;
+                    os.yx[q] = f2_add(base.yx[q], dyx);
+                    os.yz[q] = f2_add(base.yz[q], dyz);
                     ov.v[q] = va.v[q];
                 } else {
-                    os.yx[q] = cr * (in ? syx : base.yx[q]);
-                    os.yz[q] = (cr * (in ? syz : base.yz[q])) * m.sm[q];
-                    ov.v[q] = cr * va.v[q];
+                    dyx = clip(dyx, q, rm); dyz = clip(dyz, q, rm);
+                    os.yx[q] = f2_mul(c, f2_add(base.yx[q], dyx), nz2);
+                    os.yz[q] = f2_mul(f2_mul(c, f2_add(base.yz[q], dyz), nz2), m.sm[q], nz2);
+                    ov.v[q] = f2_mul(c, va.v[q], nz2);
                 }
             }
         }
@@ -468,11 +522,11 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                              Vel &ov) {
         float nu = 0.f, nw = 0.f, nv = 0.f;
         if constexpr (DIR == 0) {
-            if constexpr (PSV) { nu = __shfl_down_sync(FULL, va.u[0], 1); nw = __shfl_down_sync(FULL, va.w[0], 1); }
-            if constexpr (SH) nv = __shfl_down_sync(FULL, va.v[0], 1);
+            if constexpr (PSV) { nu = __shfl_down_sync(FULL, f2_lo(va.u[0]), 1); nw = __shfl_down_sync(FULL, f2_lo(va.w[0]), 1); }
+            if constexpr (SH) nv = __shfl_down_sync(FULL, f2_lo(va.v[0]), 1);
         } else {
-            if constexpr (PSV) { nu = __shfl_up_sync(FULL, va.u[VEC - 1], 1); nw = __shfl_up_sync(FULL, va.w[VEC - 1], 1); }
-            if constexpr (SH) nv = __shfl_up_sync(FULL, va.v[VEC - 1], 1);
+            if constexpr (PSV) { nu = __shfl_up_sync(FULL, f2_hi(va.u[NP - 1]), 1); nw = __shfl_up_sync(FULL, f2_hi(va.w[NP - 1]), 1); }
+            if constexpr (SH) nv = __shfl_up_sync(FULL, f2_hi(va.v[NP - 1]), 1);
         }
         if (all_in(r) && all_far(r) && p.surface == nullptr)
             stress_cells(std::true_type{}, r, va, vb, base, m, os, ov, nu, nw, nv);
@@ -492,24 +546,25 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                 const int q = en.x - c0;
                 if (q < 0 || q >= VEC) continue;
                 const size_t ti = (size_t)t * p.nrec_total + en.y;
-#pragma unroll
-                for (int qq = 0; qq < VEC; ++qq) {
-                    if (qq != q) continue;
-                    if constexpr (PSV) { st_chk(p.seis[0] + ti, v.u[qq]); st_chk(p.seis[2] + ti, v.w[qq]); }
-                    if constexpr (SH) st_chk(p.seis[1] + ti, v.v[qq]);
-                }
+                auto pick = [&](const f2 (&x)[NP]) {
+                    const f2 t = NP == 1 || q < 2 ? x[0] : x[NP - 1];
+                    return q & 1 ? f2_hi(t) : f2_lo(t);
+                };
+                if constexpr (PSV) { st_chk(p.seis[0] + ti, pick(v.u)); st_chk(p.seis[2] + ti, pick(v.w)); }
+                if constexpr (SH) st_chk(p.seis[1] + ti, pick(v.v));
             }
             if (k >= 0) {
                 const long long o = ((long long)p.nsnap * sh.row_off + (long long)k * nx + r) * P + c0 + COL_OFF;
-                if constexpr (PSV) { stv<VEC>(p.snap[0] + o, v.u); stv<VEC>(p.snap[2] + o, v.w); }
-                if constexpr (SH) stv<VEC>(p.snap[1] + o, v.v);
+                if constexpr (PSV) { stp<NP>(p.snap[0] + o, v.u); stp<NP>(p.snap[2] + o, v.w); }
+                if constexpr (SH) stp<NP>(p.snap[1] + o, v.v);
             }
         } else {
             if (k >= 0) {
                 const long long o = ((long long)p.nsnap * sh.row_off + (long long)k * nx + r) * P + c0 + COL_OFF;
                 const long long io = (sh.row_off + r) * (long long)P + c0 + COL_OFF;
-                auto image = [&](int c, const float (&ov)[VEC]) {
-                    float s[VEC], sum[VEC], cmp[VEC];
+                auto image = [&](int c, const f2 (&ov2)[NP]) {
+                    float s[VEC], sum[VEC], cmp[VEC], ov[VEC];
+                    unpack<NP>(ov, ov2);
                     ldv<VEC>(s, p.snap[c] + o);
                     ldv_coherent<VEC>(sum, p.img[c] + io);
                     ldv_coherent<VEC>(cmp, p.imgc[c] + io);
@@ -527,49 +582,51 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     int code = 0;
     auto check_row = [&](const Vel &v) {
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) {
-            if constexpr (PSV) {
-                code = max(code, bad_code(v.u[q], p.code_base));
-                code = max(code, bad_code(v.w[q], p.code_base + 2));
-            }
-            if constexpr (SH) code = max(code, bad_code(v.v[q], p.code_base + 1));
+        for (int q = 0; q < NP; ++q) {
+            auto bad = [&](f2 x, int c) { code = max(code, max(bad_code(f2_lo(x), c), bad_code(f2_hi(x), c))); };
+            if constexpr (PSV) { bad(v.u[q], p.code_base); bad(v.w[q], p.code_base + 2); }
+            if constexpr (SH) bad(v.v[q], p.code_base + 1);
         }
     };
     // step A's stress and absorbed velocity of row r (STOREA)
     auto store_a = [&](int r, const Sig &os, const Vel &ov) {
         const long long so = soff + (long long)(r + 1) * P;
         if constexpr (PSV) {
-            stv<VEC>(p.souta[F_SXX] + so, os.xx);
-            stv<VEC>(p.souta[F_SZZ] + so, os.zz);
-            stv<VEC>(p.souta[F_SXZ] + so, os.xz);
-            stv<VEC>(p.souta[F_U] + so, ov.u);
-            stv<VEC>(p.souta[F_W] + so, ov.w);
+            stp<NP>(p.souta[F_SXX] + so, os.xx);
+            stp<NP>(p.souta[F_SZZ] + so, os.zz);
+            stp<NP>(p.souta[F_SXZ] + so, os.xz);
+            stp<NP>(p.souta[F_U] + so, ov.u);
+            stp<NP>(p.souta[F_W] + so, ov.w);
         }
         if constexpr (SH) {
-            stv<VEC>(p.souta[F_SYX] + so, os.yx);
-            stv<VEC>(p.souta[F_SYZ] + so, os.yz);
-            stv<VEC>(p.souta[F_V] + so, ov.v);
+            stp<NP>(p.souta[F_SYX] + so, os.yx);
+            stp<NP>(p.souta[F_SYZ] + so, os.yz);
+            stp<NP>(p.souta[F_V] + so, ov.v);
         }
     };
     (void)store_a;
     // step B's stress and absorbed velocity of row r: store, outputs, check
     auto finish_b = [&](int r, const Sig &os, const Vel &ov) {
-        if constexpr (CKPT)
+        if constexpr (CKPT) {
+            float u[VEC], w[VEC], xx[VEC], zz[VEC], xz[VEC];
+            unpack<NP>(u, ov.u); unpack<NP>(w, ov.w);
+            unpack<NP>(xx, os.xx); unpack<NP>(zz, os.zz); unpack<NP>(xz, os.xz);
             ckpt_pack_row<VEC>(p.ck, soff + (long long)(r + 1) * P, ck_blk0 + (long long)(r + 1) * p.ck.nblk, lane,
-                               owner, ov.u, ov.w, os.xx, os.zz, os.xz);
+                               owner, u, w, xx, zz, xz);
+        }
         if (!owner) return;
         const long long so = soff + (long long)(r + 1) * P;
         if constexpr (PSV) {
-            stv<VEC>(p.sout[F_SXX] + so, os.xx);
-            stv<VEC>(p.sout[F_SZZ] + so, os.zz);
-            stv<VEC>(p.sout[F_SXZ] + so, os.xz);
-            stv<VEC>(p.sout[F_U] + so, ov.u);
-            stv<VEC>(p.sout[F_W] + so, ov.w);
+            stp<NP>(p.sout[F_SXX] + so, os.xx);
+            stp<NP>(p.sout[F_SZZ] + so, os.zz);
+            stp<NP>(p.sout[F_SXZ] + so, os.xz);
+            stp<NP>(p.sout[F_U] + so, ov.u);
+            stp<NP>(p.sout[F_W] + so, ov.w);
         }
         if constexpr (SH) {
-            stv<VEC>(p.sout[F_SYX] + so, os.yx);
-            stv<VEC>(p.sout[F_SYZ] + so, os.yz);
-            stv<VEC>(p.sout[F_V] + so, ov.v);
+            stp<NP>(p.sout[F_SYX] + so, os.yx);
+            stp<NP>(p.sout[F_SYZ] + so, os.yz);
+            stp<NP>(p.sout[F_V] + so, ov.v);
         }
         epilogue(r, p.it2, p.snap_k2, ov);
         if (p.check) check_row(ov);
@@ -579,8 +636,9 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     if constexpr (RING) {
         // rolling rows as in the register version below, minus 1/rho and the
         // material, which come from the ring at the point of use
-        Sig so_p, so_c, sa_p, sa_c, s_out, n_so;
-        Vel va_p, va_c, vb_p, vb_c, vo, vabs_c, vabs_p, v_out, n_vo;
+        Sig so_p, so_c, sa_p, sa_c, s_out;
+        Vel va_p, va_c, vb_p, vb_c, vo, vabs_c, vabs_p, v_out;
+        int s0 = 0, s1 = 1, s2 = 2;  // slots of state rows k, k+1, k+2
         zero_sig(sa_p); zero_sig(sa_c);
         zero_vel(va_p); zero_vel(vb_p); zero_vel(vabs_c); zero_vel(vabs_p);
         load_sig(ia - 2, so_p);
@@ -588,19 +646,17 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             // iteration k: A velocity k, A stress k-1, B velocity k-1, B stress k-2;
             // ring rows read: k (1/rho), k-1 (1/rho, material), k-2 (material);
             // issued: row k+1 into the slot of row k-3
-            load_sig(ia - 1, n_so);
-            load_vel(ia - 1, n_vo);
+            // copy groups in order: material k, state k+1, material k+1, state k+2
             ring_issue(ia - 2);
+            state_issue(0, ia - 1, ia - 1);
             ring_issue(ia - 1);
+            state_issue(1, ia, ia);
             for (int k = ia - 1; k <= ib + 1; ++k) {
-                cp_sig(so_c, n_so);
-                cp_vel(vo, n_vo);
-                if (k <= ib) {
-                    load_sig(k + 1, n_so);
-                    load_vel(k + 1, n_vo);
-                }
                 ring_issue(k + 1);
-                cp_async_wait<1>();  // every row up to k has landed
+                state_issue(s2, k + 2, k + 2);
+                cp_async_wait<3>();  // material and state up to row k have landed
+                rd_state(s0, so_c, vo);
+                { const int t = s0; s0 = s1; s1 = s2; s2 = t; }
                 {
                     Vel ir;
                     ring_ir(k, ir);
@@ -634,18 +690,15 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
         } else {
             // iteration k: A velocity k-1, A stress k-1, B velocity k-2, B stress k-2;
             // ring rows read: k-1, k-2; issued: row k into the slot of row k-4
-            load_sig(ia - 1, n_so);
-            load_vel(ia - 2, n_vo);
+            state_issue(0, ia - 1, ia - 2);
             ring_issue(ia - 2);
+            state_issue(1, ia, ia - 1);
             for (int k = ia - 1; k <= ib + 1; ++k) {
-                cp_sig(so_c, n_so);   // row k
-                cp_vel(vo, n_vo);     // row k-1
-                if (k <= ib) {
-                    load_sig(k + 1, n_so);
-                    load_vel(k, n_vo);
-                }
                 ring_issue(k);
-                cp_async_wait<1>();  // every row up to k-1 has landed
+                state_issue(s2, k + 2, k + 1);
+                cp_async_wait<3>();  // material up to row k-1, state up to row k have landed
+                rd_state(s0, so_c, vo);  // stress of row k, velocity of row k-1
+                { const int t = s0; s0 = s1; s1 = s2; s2 = t; }
                 {
                     Vel ir;
                     ring_ir(k - 1, ir);

@@ -63,6 +63,7 @@ struct ShotDev {
 struct StepParams {
     int nz, pitch, nt, fw;
     float dt, inv_dx, inv_dz, src_factor;
+    float neg_zero;        // -0.0f, opaque to the compiler (f32x2.cuh)
     const float *sponge;   // fw floats, profile by distance d = 0..fw-1
     const int4 *work;      // (shot, strip, ia, ib) per warp task
     int n_work;
