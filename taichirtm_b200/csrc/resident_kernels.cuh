@@ -659,21 +659,44 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                 if constexpr (SH) st2(p.snap[1], o + r * P, V[r]);
             }
         } else {
+            // Kahan update of G rows at a time, all their loads before the first
+            // store: one L2 round trip instead of one per row and component (the
+            // loads cannot be moved over the stores).  301 x 151, an image at every
+            // step: 2.70 -> 2.41 ms per 500-step RTM.
+            constexpr int G = R <= 2 ? 2 : 1;
             const long long io = (info->row_off + row0) * P + col + COL_OFF;
-            auto image = [&](int c, f2 v, int r) {
-                const f2 s = ld2(p.snap[c], o + r * P);
-                const f2 a = ld2(p.img[c], io + r * P), b = ld2(p.imgc[c], io + r * P);
-                float s0 = f2_lo(a), c0 = f2_lo(b), s1 = f2_hi(a), c1 = f2_hi(b);
-                kahan_add(s0, c0, __fmul_rn(f2_lo(s), f2_lo(v)));
-                kahan_add(s1, c1, __fmul_rn(f2_hi(s), f2_hi(v)));
-                st2(p.img[c], io + r * P, f2_pack(s0, s1));
-                st2(p.imgc[c], io + r * P, f2_pack(c0, c1));
-            };
+            constexpr int NCI = (PSV ? 2 : 0) + (SH ? 1 : 0);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (!(own >> r & 1)) continue;
-                if constexpr (PSV) { image(0, U[r], r); image(2, W[r], r); }
-                if constexpr (SH) image(1, V[r], r);
+            for (int r0 = 0; r0 < R; r0 += G) {
+                f2 sn[G][NCI], im[G][NCI], ic[G][NCI];
+#pragma unroll
+                for (int h = 0; h < G; ++h)
+#pragma unroll
+                    for (int c = 0; c < NCI; ++c) {
+                        const int comp = !PSV ? 1 : c == 0 ? 0 : c == 1 ? 2 : 1;
+                        const int r = r0 + h;
+                        if (r >= R || !(own >> r & 1)) continue;
+                        sn[h][c] = ld2(p.snap[comp], o + r * P);
+                        im[h][c] = ld2(p.img[comp], io + r * P);
+                        ic[h][c] = ld2(p.imgc[comp], io + r * P);
+                    }
+#pragma unroll
+                for (int h = 0; h < G; ++h)
+#pragma unroll
+                    for (int c = 0; c < NCI; ++c) {
+                        const int comp = !PSV ? 1 : c == 0 ? 0 : c == 1 ? 2 : 1;
+                        const int r = r0 + h;
+                        if (r >= R || !(own >> r & 1)) continue;
+                        f2 v;
+                        if constexpr (PSV && SH) v = c == 0 ? U[r] : c == 1 ? W[r] : V[r];
+                        else if constexpr (PSV) v = c == 0 ? U[r] : W[r];
+                        else v = V[r];
+                        float s0 = f2_lo(im[h][c]), c0 = f2_lo(ic[h][c]), s1 = f2_hi(im[h][c]), c1 = f2_hi(ic[h][c]);
+                        kahan_add(s0, c0, __fmul_rn(f2_lo(sn[h][c]), f2_lo(v)));
+                        kahan_add(s1, c1, __fmul_rn(f2_hi(sn[h][c]), f2_hi(v)));
+                        st2(p.img[comp], io + r * P, f2_pack(s0, s1));
+                        st2(p.imgc[comp], io + r * P, f2_pack(c0, c1));
+                    }
             }
         }
     };
