@@ -41,4 +41,32 @@ static __global__ void ckpt_unpack_kernel(CkptIn ci) {
     }
 }
 
+// Store of a whole FP32 state (of a resident launch) into a compressed slot:
+// one warp per row, field and block of 60 columns, the block as the two
+// columns per lane of ckpt_pack_field<2>, so the slot's bits are those that a
+// storing step launch writes.  Shots that stopped before step seq are left out.
+// grid: (chunks, nshots, 5 fields)
+struct CkptFrom {
+    const float *src[5];       // u, w, sxx, szz, sxz
+    const ShotDev *shots;
+    const int *fail_seq;
+    int pitch, nz, seq;
+};
+static __global__ void ckpt_pack_kernel(CkptOut ck, CkptFrom from) {
+    const int shot = blockIdx.y, f = blockIdx.z, lane = threadIdx.x & 31;
+    if (from.fail_seq[shot] < from.seq) return;
+    const ShotDev sh = from.shots[shot];
+    const long long row0 = sh.state_off / from.pitch;  // padded row 0 of the shot
+    const int warps = gridDim.x * (blockDim.x >> 5);
+    for (long long k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < (long long)sh.nx * ck.nblk; k += warps) {
+        const int i = (int)(k / ck.nblk), b = (int)(k % ck.nblk), j = 60 * b - 2 + 2 * lane;
+        const bool owner = lane >= 1 && lane <= 30;
+        const long long e = sh.state_off + (long long)(i + 1) * from.pitch + j + COL_OFF;
+        float v[2] = {0.f, 0.f};
+        if (owner && j < from.nz) v[0] = ldg_chk(from.src[f] + e);
+        if (owner && j + 1 < from.nz) v[1] = ldg_chk(from.src[f] + e + 1);
+        ckpt_pack_field<2>(ck, f, e, (row0 + i + 1) * ck.nblk + b, lane, owner, v);
+    }
+}
+
 }  // namespace rtm

@@ -63,7 +63,8 @@ struct ResParams {
     // loop: steps it0 .. it1-1; the time of step it is it (forward) or nt-1-it (backward)
     int it0, it1, check_interval;
     int isnap, snap_base, snap_lo, snap_hi;  // time t = m * isnap, m in [snap_lo, snap_hi]: slot m - snap_base
-    // state: loaded from load[] (null: zero), owned cells stored to store[] at the end
+    bool segment;              // part of a loop: shots stopped earlier are left alone
+    // state: loaded from load[] (null: zero), owned cells stored to store[] at the end (null: not)
     const float *load[NFIELD];
     float *store[NFIELD];
     // tiles
@@ -217,6 +218,8 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
         const int nx = sh.nx, nz = p.nz, P = p.pitch;
         constexpr int H = RES_HALO;
         const int row0 = tl.y - H + warp * R, col = tl.z - H + 2 * lane;
+        // a failure of this launch is later than it0, so all tiles agree
+        if (p.segment && ld_acquire(p.fail_seq + tl.x) <= p.it0) return;
         if (threadIdx.x == 0) {
             info->state_off = sh.state_off;
             info->row_off = sh.row_off;
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
         };
         for (int rr = threadIdx.x; rr < RT; rr += 32 * NW) {
             s_ip[rr] = row_entries(inj_ptr, inj_ent, rr, false, nullptr, 0);
-            if (DIR == 0) s_rp[rr] = row_entries(p.rec_ptr + sh.rec_row0, p.rec_ent, rr, true, nullptr, 0);
+            if (DIR == 0) s_rp[rr] = p.seis[PSV ? 0 : 1] ? row_entries(p.rec_ptr + sh.rec_row0, p.rec_ent, rr, true, nullptr, 0) : 0;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -332,7 +335,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
             row_entries(inj_ptr, inj_ent, rr, false, s_inj + a, n);
             const int b = DIR == 0 ? s_rp[rr] : a, m = DIR == 0 ? s_rp[rr + 1] - b : n;
             const int2 *ent = DIR == 0 ? s_rec() + b : s_inj + a;
-            if (DIR == 0) row_entries(p.rec_ptr + sh.rec_row0, p.rec_ent, rr, true, s_rec() + b, m);
+            if (DIR == 0 && m) row_entries(p.rec_ptr + sh.rec_row0, p.rec_ent, rr, true, s_rec() + b, m);
             unsigned short *t = s_pt + rr * 32;
             for (int l = 0; l < 32; ++l) t[l] = RES_NONE;
             for (int e = 0; e < m; ++e) {
@@ -925,8 +928,8 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
         }
     }
     cp_async_wait<0>();
-    // final state of the owned cells
-    {
+    // final state of the owned cells; a shot that stopped inside a segment leaves none
+    if (p.store[PSV ? F_U : F_V] && !(p.segment && info->leave == 2 && it < p.it1)) {
         const int row0 = my_row0(), col = my_col();
         if (!lane_owned(col)) return;
         const unsigned own = rows_own(row0, info->nx);

@@ -163,6 +163,7 @@ struct rtm_plan {
         int *d_sync = nullptr;   // checks passed per shot
         uint4 *d_box = nullptr;  // outboxes of the largest launch
         size_t box_bytes = 0;
+        unsigned tag = 0;        // tags used by the current call
         std::vector<int2> waves;  // (first tile, tiles) of each launch
         void *base = nullptr;     // their allocation
     } res;
@@ -653,15 +654,22 @@ void resident_params(const rtm_plan *p, ResParams &rp, int dir) {
     rp.max_rec = dir == 0 ? p->res.max_rec : 0;
 }
 
+// Before the first resident_run of a call: no packet carries tag 0, and the tags
+// then go on from run to run.
+int resident_begin(rtm_plan *p, cudaStream_t s) {
+    CUDA_TRY(cudaMemsetAsync(p->res.d_box, 0, p->res.box_bytes, s));
+    p->res.tag = 0;
+    return 0;
+}
+
 // Run the loop of rp for every shot, wave by wave.
 int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
     CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
-    CUDA_TRY(cudaMemsetAsync(p->res.d_box, 0, p->res.box_bytes, s));  // no packet carries tag 0
-    rp.tag0 = 0;
     const unsigned blocks = (unsigned)resident_blocks(rp.it0, rp.it1, rp.check_interval);
     const size_t smem = resident_smem(p, p->res.r, p->res.warps, rp.max_inj, rp.max_rec, p->res.surface);
     for (const int2 &w : p->res.waves) {
         rp.tile0 = w.x;
+        rp.tag0 = p->res.tag;
         cudaError_t e = cudaErrorInvalidValue;
         auto go = [&](auto d, auto m, auto r, auto n) {
             void *args[] = {&rp};
@@ -672,7 +680,7 @@ int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
         else res_dispatch<1>(p->g.modes, p->res.r, p->res.warps, go);
         CUDA_TRY(e);
         ++p->launches;
-        rp.tag0 += blocks;
+        p->res.tag += blocks;
     }
     return 0;
 }
@@ -1238,6 +1246,7 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
             rp.snap_base = rp.snap_lo = 1;
             rp.snap_hi = nsnap;
         }
+        if (int rc = resident_begin(p, s)) return rc;
         if (int rc = resident_run(p, rp, 0, s)) return rc;
         p->live = 0;
     } else if (p->cb) {  // host callbacks in the loop: direct launches
@@ -1378,6 +1387,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
             rp.snap_base = rp.snap_lo = 1;
             rp.snap_hi = num_snaps;
         }
+        if (int rc = resident_begin(p, s)) return rc;
         if (int rc = resident_run(p, rp, 1, s)) return rc;
         p->live = 0;
     } else if (p->cb) {  // host callbacks in the loop: direct launches
@@ -1541,6 +1551,21 @@ int ckpt_load(rtm_plan *p, const void *ckpt, int dtype, int c, float *const *dst
     return 0;
 }
 
+// Pack the FP32 state src[] (after step seq - 1) into compressed slot c.
+int ckpt_store(rtm_plan *p, void *ckpt, int dtype, int c, float *const *src, int seq, cudaStream_t s) {
+    CkptFrom from{};
+    for (int f = 0; f < NADJ; ++f) from.src[f] = src[f];
+    from.shots = p->d_shots;
+    from.fail_seq = p->d_fail_seq;
+    from.pitch = p->pitch;
+    from.nz = p->g.nz;
+    from.seq = seq;
+    ckpt_pack_kernel<<<dim3(64, p->nshots, NADJ), 256, 0, s>>>(ckpt_out(p, ckpt, dtype, c), from);
+    CUDA_TRY(cudaGetLastError());
+    ++p->launches;
+    return 0;
+}
+
 // Where segment sgi's start state (after step sgi*K - 1) lives: the zero
 // state for sgi = 0, the FP32 slot itself, or `stage` after unpacking.
 int segment_start(rtm_plan *p, const void *ckpt, int dtype, int sgi, float *zero, float *stage,
@@ -1581,7 +1606,8 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
     bs.add(seis, (size_t)3 * p->nrec_total * nt * sizeof(float));
     bs.add(ckpt, rtm_plan_checkpoint_bytes(p, ckpt_every, ckpt_dtype));
     if (int rc = bs.begin(s)) return rc;
-    if (int rc = zero_state(p, s)) return rc;
+    const bool resident = p->res.r > 0;
+    if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
     // every slot starts at zero: pad rows / columns of FP32 slots, and the
     // slots of a shot that stops before reaching them
     if (nck > 0) CUDA_TRY(cudaMemsetAsync(ckpt, 0, rtm_plan_checkpoint_bytes(p, ckpt_every, ckpt_dtype), s));
@@ -1601,8 +1627,38 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
     p->live = -1;
     auto check_at = [&](int it) { return check_interval > 0 && it % check_interval == 0; };
     auto save_at = [&](int it) { return (it + 1) % ckpt_every == 0 && it + 1 < nt; };
+    if (resident) {
+        // one segment between checkpoints at a time, its end state stored in FP32:
+        // straight into an FP32 slot, or into a state buffer and packed from there
+        ResParams rp;
+        resident_params(p, rp, 0);
+        for (int c = 0; c < 3; ++c) {
+            rp.wav[c] = sp.wav[c];
+            rp.seis[c] = sp.seis[c];
+        }
+        rp.code_base = 1;
+        rp.check_interval = check_interval;
+        rp.segment = true;
+        if (int rc = resident_begin(p, s)) return rc;
+        for (int start = 0, seg = 0; start < nt; start += ckpt_every, ++seg) {
+            const int end = std::min(start + ckpt_every, nt);
+            const bool save = end < nt, f32 = ckpt_dtype == RTM_CKPT_F32;
+            float *dst[NADJ];
+            for (int f = 0; f < NADJ; ++f)
+                dst[f] = save && f32 ? reinterpret_cast<float *>(ckpt_slot(p, ckpt, ckpt_dtype, seg)) + (size_t)f * p->state_floats
+                                     : p->d_state[seg & 1][f];
+            for (int f = 0; f < NADJ; ++f) rp.store[f] = save ? dst[f] : nullptr;
+            rp.it0 = start;
+            rp.it1 = end;
+            if (int rc = resident_run(p, rp, 0, s)) return rc;
+            if (save && !f32) {
+                if (int rc = ckpt_store(p, ckpt, ckpt_dtype, seg, dst, end, s)) return rc;
+            }
+            for (int f = 0; f < NADJ; ++f) rp.load[f] = dst[f];
+        }
+    }
     const std::vector<LoopLaunch> sched =
-        loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !save_at(it); });
+        resident ? std::vector<LoopLaunch>() : loop_schedule(0, nt, p->tsteps, [&](int it) { return !check_at(it) && !save_at(it); });
     for (const LoopLaunch &ln : sched) {
         const int last = ln.two ? ln.it + 1 : ln.it;  // the step whose state the launch writes
         const bool save = save_at(last);
@@ -1639,10 +1695,8 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
         if (int rc = transpose(p->d_seis_t, seis, 3, nt, p->nrec_total, s)) return rc;
         ++p->launches;
     }
-    if (flags) {
-        CUDA_TRY(cudaMemcpyAsync(flags, p->d_flags, p->nshots * sizeof(int), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(cudaStreamSynchronize(s));
-    }
+    if (flags)
+        if (int rc = read_status(p, flags, s)) return rc;
     if (int rc = bs.end(s)) return rc;
     return RTM_OK;
 }
@@ -1887,8 +1941,10 @@ int rtm_backward_checkpointed(rtm_plan *p, const float *wavelets, const float *o
     p->live = -1;
     auto body = [&]() -> int {
         if (int rc = bs.begin(s)) return rc;
-        if (int rc = zero_state(p, s)) return rc;
-        CUDA_TRY(cudaMemsetAsync(buf, 0, nbuf * sizeof(float), s));
+        const bool resident = p->res.r > 0;
+        if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
+        if (!resident) CUDA_TRY(cudaMemsetAsync(buf, 0, nbuf * sizeof(float), s));
+        else if (int rc = resident_begin(p, s)) return rc;
         const size_t img_floats = (size_t)p->rows_total * p->pitch;
         for (int c = 0; c < 3; ++c)
             if (p->d_img[c]) {
@@ -1936,6 +1992,50 @@ int rtm_backward_checkpointed(rtm_plan *p, const float *wavelets, const float *o
             // recompute forward steps start .. end-1, keeping u, w at imaging steps
             const int first = ((start + isnap - 1) / isnap) * isnap;  // first multiple of isnap >= start
             auto slot_at = [&](int t) { return images_at(t) ? (t - first) / isnap : -1; };
+            if (resident) {
+                ResParams rp;
+                resident_params(p, rp, 0);
+                for (int c = 0; c < 3; ++c) rp.wav[c] = fp.wav[c];
+                rp.nsnap = seg_snaps;
+                rp.snap[0] = snapu;
+                rp.snap[2] = snapw;
+                rp.isnap = isnap;
+                rp.snap_base = first / isnap;
+                rp.snap_lo = 1;
+                rp.snap_hi = num_snaps;
+                rp.it0 = start;
+                rp.it1 = end;
+                for (int f = 0; f < NADJ; ++f) {
+                    rp.load[f] = sgi == 0 ? nullptr : s0 + (size_t)f * sf;
+                    rp.store[f] = nullptr;
+                }
+                if (int r = resident_run(p, rp, 0, s)) return r;
+                resident_params(p, rp, 1);
+                for (int c = 0; c < 3; ++c) {
+                    rp.obs[c] = bp.obs[c];
+                    rp.img[c] = bp.img[c];
+                    rp.imgc[c] = bp.imgc[c];
+                }
+                rp.nsnap = seg_snaps;
+                rp.snap[0] = snapu;
+                rp.snap[2] = snapw;
+                rp.isnap = isnap;
+                rp.snap_base = first / isnap;
+                rp.snap_lo = 1;
+                rp.snap_hi = num_snaps;
+                rp.code_base = 4;
+                rp.check_interval = check_interval;
+                rp.segment = true;
+                rp.it0 = nt - end;
+                rp.it1 = nt - start;
+                for (int f = 0; f < NADJ; ++f) {
+                    rp.load[f] = nb == 0 ? nullptr : p->d_state[nb & 1][f];
+                    rp.store[f] = p->d_state[(nb + 1) & 1][f];
+                }
+                if (int r = resident_run(p, rp, 1, s)) return r;
+                ++nb;
+                continue;
+            }
             const std::vector<LoopLaunch> fsched = loop_schedule(start, end, p->tsteps, [](int) { return true; });
             for (size_t L = 0; L < fsched.size(); ++L) {
                 const int it = fsched[L].it;
@@ -2005,8 +2105,8 @@ int rtm_backward_checkpointed(rtm_plan *p, const float *wavelets, const float *o
                     CUDA_TRY(cudaGetLastError());
                 }
         }
-        if (flags) CUDA_TRY(cudaMemcpyAsync(flags, p->d_flags, p->nshots * sizeof(int), cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(cudaStreamSynchronize(s));
+        std::vector<int32_t> status(p->nshots);  // the call waits for its results in any case
+        if (int rc = read_status(p, flags ? flags : status.data(), s)) return rc;
         if (int rc = bs.end(s)) return rc;
         return RTM_OK;
     };

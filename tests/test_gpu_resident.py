@@ -128,3 +128,36 @@ def test_failing_shots_stop_at_the_same_check(check):
     a = _run(shots, nx, nz, nt, 10, 3, None, wav, 2, check, resident=True)
     assert a[0][0] > 0 and a[0][1] == 0
     _same(a, _run(shots, nx, nz, nt, 10, 3, STREAM, wav, 2, check))
+
+
+@pytest.mark.parametrize("store", ["f32", "f16", "bf16", "i16"])
+@pytest.mark.parametrize("every,nt,isnap,check", [(1, 7, 2, 0), (5, 23, 1, 4), (8, 24, 3, 8), (40, 23, 4, 5)])
+def test_checkpointed_segments(store, every, nt, isnap, check):
+    """Checkpoint slots, seismograms and the image of checkpointed RTM, and the
+    gradient from those checkpoints, equal the streaming kernels' (vec 2)."""
+    import ctypes
+    from taichirtm_b200 import _lib
+    from taichirtm_b200.plan import Plan, ShotGeometry, _i32p, _ptr, _stream, check as ok
+    nx, nz, fw = 230, 131, 12
+    shots = [ShotGeometry(0, 121, *_points(121, nz, dense=True)), ShotGeometry(99, 131, *_points(131, nz, dense=False))]
+    wav = torch.as_tensor(_wavelets(sum(len(s.src) for s in shots), nt)).cuda()
+    L, dt, res = _lib.lib(), _lib.CKPT_DTYPES[store], []
+    for tune in (None, dict(vec=2, rows=9, warps=2, tsteps=2)):
+        p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, fw, 1, shots, tune=tune)
+        p.set_model(*_model(nx, nz))
+        assert p.resident() == (tune is None)
+        ck = torch.zeros(max(int(L.rtm_plan_checkpoint_bytes(p.h, every, dt)), 1), dtype=torch.uint8, device="cuda")
+        seis = torch.zeros((3, p.nrec_total, nt), device="cuda")
+        stack = torch.zeros((3, nx, nz), dtype=torch.float64, device="cuda")
+        grad = torch.zeros((5, nx, nz), dtype=torch.float64, device="cuda")
+        flags, flags_b = np.zeros(2, np.int32), np.zeros(2, np.int32)
+        ok(L.rtm_forward_checkpointed(p.h, _ptr(wav), _ptr(seis), every, dt, _ptr(ck), check, _i32p(flags), _stream()), "f")
+        obs = (seis * 0.5 + 1e-3).contiguous()
+        ok(L.rtm_backward_checkpointed(p.h, _ptr(wav), _ptr(obs), every, dt, _ptr(ck), isnap, None, _ptr(stack), check,
+                                       _i32p(flags_b), _stream()), "b")
+        ok(L.rtm_adjoint(p.h, _ptr(wav), _ptr(obs), every, dt, _ptr(ck), _ptr(grad), ctypes.c_void_p(0), _stream()), "a")
+        # FP32 slots are compared through the image and the gradient read from them
+        res.append([flags, flags_b] + [x.cpu().numpy() for x in (seis, stack, grad)] + ([ck.cpu().numpy()] if dt else []))
+        p.close()
+    assert np.abs(res[0][3]).max() > 0 and np.abs(res[0][4]).max() > 0
+    _same(*res)
