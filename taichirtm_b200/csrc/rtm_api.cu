@@ -369,11 +369,11 @@ cudaError_t launch_step2(const StepParams &sp, int warps, cudaStream_t s) {
     size_t smem = 0;
     if constexpr (RING) {
         constexpr size_t kMaxSmem = 227 * 1024;  // per-block opt-in limit
-        smem = (size_t)warps * ring2_smem_per_warp<MODE, VEC>(sp.surface != nullptr);
+        smem = (size_t)warps * ring2_smem_per_warp<DIR, MODE, VEC>(sp.surface != nullptr);
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
         static bool attr_set = false;  // per instantiation; raises the 48 KB default
         if (!attr_set) {
-            const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<MODE, VEC>(true), kMaxSmem);
+            const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<DIR, MODE, VEC>(true), kMaxSmem);
             cudaError_t e = cudaFuncSetAttribute(step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
             if (e != cudaSuccess) return e;
@@ -892,6 +892,15 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
         while (p->rows > 1 && rows_all / p->rows * strips < 148 * 16) p->rows /= 2;
         p->warps = 4;
         p->prefetch = p->rows >= 12 ? 3 : 1;
+        // Long lists of tasks run fastest with 4 columns per lane, one warp per CTA
+        // (14 windows of about 800 x 716, both wave types: 71 against 100 us per
+        // step).  P-SV plans may be asked for an adjoint, which 2 columns suit.
+        if (g.modes != RTM_PSV && rows_all / 24 * ((g.nz + 119) / 120) >= 148 * 12) {
+            p->vec = 4;
+            p->rows = 24;
+            p->warps = 1;
+            p->prefetch = 4;
+        }
     }
     const int W = 30 * p->vec;
     p->nstrips = (g.nz + W - 1) / W;
@@ -1400,28 +1409,25 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
     const int blocks = 148 * 8;
     const size_t n = (size_t)p->g.nx * p->g.nz;
     // source illumination (rtm_backward_normalized): FP64 per cell, one
-    // component at a time, over the snapshot slots the correlation used
-    struct Scratch {
+    // component at a time, over the snapshot slots the correlation used; in the
+    // plan's scratch (allocated for each call, it took 2 to 10 ms of it)
+    struct {
         double *illum = nullptr;
         unsigned long long *imax = nullptr;
         int *slots = nullptr;
-        ~Scratch() {
-            if (illum) cudaFree(illum);
-            if (imax) cudaFree(imax);
-            if (slots) cudaFree(slots);
-        }
     } sc;
     std::vector<int> slots;
     const bool norm = norm_eps >= 0.0;
     if (norm) {
         for (int it = 0; it < nt; ++it)
             if (snap_of[it] >= 0) slots.push_back(snap_of[it]);
-        if (int rc = dalloc(&sc.illum, img_floats)) return rc;
-        if (int rc = dalloc(&sc.imax, (size_t)p->nshots)) return rc;
-        if (!slots.empty()) {
-            if (int rc = dalloc(&sc.slots, slots.size())) return rc;
+        float *scratch = nullptr;
+        if (int rc = plan_scratch(p, 2 * (img_floats + (size_t)p->nshots) + slots.size(), &scratch)) return rc;
+        sc.illum = reinterpret_cast<double *>(scratch);
+        sc.imax = reinterpret_cast<unsigned long long *>(sc.illum + img_floats);
+        sc.slots = reinterpret_cast<int *>(sc.imax + p->nshots);
+        if (!slots.empty())
             CUDA_TRY(cudaMemcpyAsync(sc.slots, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-        }
     }
     for (int c = 0; c < 3; ++c) {
         IllumNorm nm;
@@ -1456,7 +1462,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
     if (flags) {
         if (int rc = read_status(p, flags, s)) return rc;
     } else if (norm) {
-        CUDA_TRY(cudaStreamSynchronize(s));  // scratch is freed on return
+        CUDA_TRY(cudaStreamSynchronize(s));  // the slot table is host memory of this call
     }
     if (int rc = bs.end(s)) return rc;
     return RTM_OK;
