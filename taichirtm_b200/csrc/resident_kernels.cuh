@@ -68,10 +68,11 @@ struct ResParams {
     const float *load[NFIELD];
     float *store[NFIELD];
     // tiles
-    const int4 *tiles;         // (shot, first owned row, first owned column, unused); a shot's tiles row by row
-    const int4 *shot_tiles;    // per shot: (unused, tile rows, tile columns, unused)
+    const int4 *tiles;         // (shot, first owned row, first owned column, wave type); a shot's tiles row by row
+    const int4 *shot_tiles;    // per shot, P-SV and SH: (tiles of the shot, tile rows, tile columns, unused)
     int tile0;                 // first tile of this launch
-    uint4 *outbox;             // per CTA of the launch: 2 x ResSmem::BOX packets
+    uint4 *outbox;             // per CTA of the launch: box_stride packets, two outboxes of ResSmem::BOX
+    int box_stride;
     unsigned tag0;             // exchange b of this launch is tagged tag0 + b
     int *arrive;               // per shot: checks passed, summed over its tiles
     int *err;
@@ -122,7 +123,8 @@ struct ResInfo {
     long long state_off, row_off;
     int nx, shot, row0, col0;  // first owned row and column
     int nti, ntj;              // the shot's tile rows and columns
-    int leave, pad;
+    int tiles;                 // tiles of the shot, of both wave types
+    int leave;
 };
 static_assert(sizeof(ResInfo) <= 64, "");
 
@@ -173,8 +175,10 @@ constexpr int res_ctas() {
     return (state <= 30 ? 32 : state <= 40 ? 24 : 16) / NW;
 }
 
+extern __shared__ __align__(16) unsigned char res_smem_raw[];
+
 template <int DIR, int MODE, int R, int NW>
-__global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_kernel(const ResParams p) {
+__device__ __forceinline__ void resident_body(const ResParams &p) {
     using L = ResSmem<MODE, R, NW>;
     constexpr bool PSV = (MODE & 1) != 0;
     constexpr bool SH = (MODE & 2) != 0;
@@ -184,7 +188,6 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
     const int lane = threadIdx.x & 31;
     const int warp = __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0);  // known to be the same on every lane
 
-    extern __shared__ __align__(16) unsigned char res_smem_raw[];
     unsigned char *const sm0 = res_smem_raw;
     volatile ResInfo *const info = reinterpret_cast<volatile ResInfo *>(sm0 + L::INFO);
     unsigned short *const s_pt = reinterpret_cast<unsigned short *>(sm0 + L::PT);
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
     int points = 0;         // receivers in this warp's rows: 0 none, 1 by the table, 2 by the lists
     {
         const int4 tl = p.tiles[p.tile0 + blockIdx.x];
-        const int4 st = p.shot_tiles[tl.x];
+        const int4 st = p.shot_tiles[2 * tl.x + (PSV ? 0 : 1)];
         const ShotDev sh = p.shots[tl.x];
         const int nx = sh.nx, nz = p.nz, P = p.pitch;
         constexpr int H = RES_HALO;
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
             info->col0 = tl.z;
             info->nti = st.y;
             info->ntj = st.z;
+            info->tiles = st.x;
             info->leave = 0;
         }
         cm0 = (unsigned)(col - 1) < (unsigned)(nz - 2) ? ~0u : 0u;
@@ -662,44 +666,52 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                 if constexpr (SH) st2(p.snap[1], o + r * P, V[r]);
             }
         } else {
-            // Kahan update of G rows at a time, all their loads before the first
-            // store: one L2 round trip instead of one per row and component (the
-            // loads cannot be moved over the stores).  301 x 151, an image at every
-            // step: 2.70 -> 2.41 ms per 500-step RTM.
-            constexpr int G = R <= 2 ? 2 : 1;
+            // Kahan update.  Two-row tiles load everything before the first store: one
+            // L2 round trip instead of one per row and component (the loads cannot be
+            // moved over the stores); 301 x 151, an image at every step: 2.70 -> 2.40 ms
+            // per 500-step RTM.  Taller ones have no registers for it: the spills
+            // cost every step (R 6: 3.0 -> 3.4 us).
             const long long io = (info->row_off + row0) * P + col + COL_OFF;
-            constexpr int NCI = (PSV ? 2 : 0) + (SH ? 1 : 0);
+            auto update = [&](int c, int r, f2 sn, f2 im, f2 ic, f2 v) {
+                float s0 = f2_lo(im), c0 = f2_lo(ic), s1 = f2_hi(im), c1 = f2_hi(ic);
+                kahan_add(s0, c0, __fmul_rn(f2_lo(sn), f2_lo(v)));
+                kahan_add(s1, c1, __fmul_rn(f2_hi(sn), f2_hi(v)));
+                st2(p.img[c], io + r * P, f2_pack(s0, s1));
+                st2(p.imgc[c], io + r * P, f2_pack(c0, c1));
+            };
+            if constexpr (R == 2) {
+                constexpr int N = PSV ? 2 : 1;
+                f2 sn[R][N], im[R][N], ic[R][N];
 #pragma unroll
-            for (int r0 = 0; r0 < R; r0 += G) {
-                f2 sn[G][NCI], im[G][NCI], ic[G][NCI];
+                for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int h = 0; h < G; ++h)
-#pragma unroll
-                    for (int c = 0; c < NCI; ++c) {
-                        const int comp = !PSV ? 1 : c == 0 ? 0 : c == 1 ? 2 : 1;
-                        const int r = r0 + h;
-                        if (r >= R || !(own >> r & 1)) continue;
-                        sn[h][c] = ld2(p.snap[comp], o + r * P);
-                        im[h][c] = ld2(p.img[comp], io + r * P);
-                        ic[h][c] = ld2(p.imgc[comp], io + r * P);
+                    for (int k = 0; k < N; ++k) {
+                        const int c = PSV ? 2 * k : 1;
+                        if (!(own >> r & 1)) continue;
+                        sn[r][k] = ld2(p.snap[c], o + r * P);
+                        im[r][k] = ld2(p.img[c], io + r * P);
+                        ic[r][k] = ld2(p.imgc[c], io + r * P);
                     }
 #pragma unroll
-                for (int h = 0; h < G; ++h)
-#pragma unroll
-                    for (int c = 0; c < NCI; ++c) {
-                        const int comp = !PSV ? 1 : c == 0 ? 0 : c == 1 ? 2 : 1;
-                        const int r = r0 + h;
-                        if (r >= R || !(own >> r & 1)) continue;
-                        f2 v;
-                        if constexpr (PSV && SH) v = c == 0 ? U[r] : c == 1 ? W[r] : V[r];
-                        else if constexpr (PSV) v = c == 0 ? U[r] : W[r];
-                        else v = V[r];
-                        float s0 = f2_lo(im[h][c]), c0 = f2_lo(ic[h][c]), s1 = f2_hi(im[h][c]), c1 = f2_hi(ic[h][c]);
-                        kahan_add(s0, c0, __fmul_rn(f2_lo(sn[h][c]), f2_lo(v)));
-                        kahan_add(s1, c1, __fmul_rn(f2_hi(sn[h][c]), f2_hi(v)));
-                        st2(p.img[comp], io + r * P, f2_pack(s0, s1));
-                        st2(p.imgc[comp], io + r * P, f2_pack(c0, c1));
+                for (int r = 0; r < R; ++r) {
+                    if (!(own >> r & 1)) continue;
+                    if constexpr (PSV) {
+                        update(0, r, sn[r][0], im[r][0], ic[r][0], U[r]);
+                        update(2, r, sn[r][1], im[r][1], ic[r][1], W[r]);
+                    } else {
+                        update(1, r, sn[r][0], im[r][0], ic[r][0], V[r]);
                     }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (!(own >> r & 1)) continue;
+                    auto image = [&](int c, f2 v) {
+                        update(c, r, ld2(p.snap[c], o + r * P), ld2(p.img[c], io + r * P), ld2(p.imgc[c], io + r * P), v);
+                    };
+                    if constexpr (PSV) { image(0, U[r]); image(2, W[r]); }
+                    if constexpr (SH) image(1, V[r]);
+                }
             }
         }
     };
@@ -764,7 +776,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                 for (int r = 0; r < R; ++r) {
                     const int rr = warp * R + r;
                     if (!(own >> r & 1) || !(side || rr < 2 * RES_HALO || rr >= RT - 2 * RES_HALO)) continue;
-                    uint4 *q = box + (size_t)blockIdx.x * (2 * L::BOX) + (rr - RES_HALO) * (L::NP * L::OLN) + ol;
+                    uint4 *q = box + (size_t)blockIdx.x * p.box_stride + (rr - RES_HALO) * (L::NP * L::OLN) + ol;
                     if (!RTM_DBG_OK(q, 16) || !RTM_DBG_OK(q + (L::NP - 1) * L::OLN, 16)) continue;
                     // packet k: pair k and one value of the pairs left over (L::place)
                     if constexpr (PSV) {
@@ -793,11 +805,11 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                 const int j = col0 - RES_HALO + 2 * ln;
                 if ((unsigned)j >= (unsigned)p.nz) return INT_MIN;
                 int pl = ln - RES_HALO / 2, d = 0;
-                if (pl < 0) { pl += L::OLN; d = -2 * L::BOX; }
-                else if (pl >= L::OLN) { pl -= L::OLN; d = 2 * L::BOX; }
+                if (pl < 0) { pl += L::OLN; d = -p.box_stride; }
+                else if (pl >= L::OLN) { pl -= L::OLN; d = p.box_stride; }
                 return d + pl;
             };
-            const uint4 *const me = box + (size_t)blockIdx.x * (2 * L::BOX);
+            const uint4 *const me = box + (size_t)blockIdx.x * p.box_stride;
             constexpr int FU = 2 * RES_HALO * L::NP, FP = (FU + NW - 1) / NW;              // whole-row units, per warp
             constexpr int G = 32 / RES_HALO, SU = (L::ORW * L::NP + G - 1) / G, SP = (SU + NW - 1) / NW;  // side units
             const int sl = lane % RES_HALO, sln = sl < RES_HALO / 2 ? sl : sl + L::OLN;
@@ -813,7 +825,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                     const bool up = hr < RES_HALO;
                     const int i = trow0 + (up ? hr : hr + L::ORW), pr = up ? L::ORW - RES_HALO + hr : hr - RES_HALO;
                     in = (FU % NW == 0 || u < FU) && lp != INT_MIN && (unsigned)i < (unsigned)nx;
-                    src[k] = me + ((up ? -ntj : ntj) * (2 * L::BOX) + (pr * L::NP + pn) * L::OLN + lp);
+                    src[k] = me + ((up ? -ntj : ntj) * p.box_stride + (pr * L::NP + pn) * L::OLN + lp);
                 } else {
                     const int m = ((k - FP) * NW + warp) * G + lane / RES_HALO, pr = m / L::NP;  // owned row; packet m % NP
                     in = m < L::ORW * L::NP && slp != INT_MIN && trow0 + RES_HALO + pr < nx;
@@ -920,7 +932,7 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
                 int *const arrive = p.arrive + info->shot;
                 __threadfence();
                 atomicAdd(arrive, 1);
-                if (!res_wait(arrive, checks * info->nti * info->ntj, p.err)) info->leave = 1;
+                if (!res_wait(arrive, checks * info->tiles, p.err)) info->leave = 1;
                 if (ld_acquire(p.fail_seq + info->shot) <= it) info->leave = 2;  // failed at this check
             }
             __syncthreads();
@@ -940,6 +952,22 @@ __global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_ker
             store_row(r, so + (long long)r * p.pitch, p.store);
         }
     }
+}
+
+template <int DIR, int MODE, int R, int NW>
+__global__ void __launch_bounds__(32 * NW, res_ctas<MODE, R, NW>()) resident_kernel(const ResParams p) {
+    resident_body<DIR, MODE, R, NW>(p);
+}
+
+// Both wave types: they never read each other's fields, so each has tiles of its
+// own, with its own rows per lane; the finite checks stop them together.  (One
+// tile for both takes 128 registers at R 2: 86 against 97 Gcell/s on a full chip,
+// and 1.85 against 1.07 us per step on 72 x 56.)
+template <int DIR, int RP, int RS, int NW>
+__global__ void __launch_bounds__(32 * NW, res_ctas<1, RP, NW>() < res_ctas<2, RS, NW>() ? res_ctas<1, RP, NW>() : res_ctas<2, RS, NW>())
+resident_both_kernel(const ResParams p) {
+    if (p.tiles[p.tile0 + blockIdx.x].w == 0) resident_body<DIR, 1, RP, NW>(p);
+    else resident_body<DIR, 2, RS, NW>(p);
 }
 
 }  // namespace rtm

@@ -156,13 +156,14 @@ struct rtm_plan {
     // Resident propagation (resident_kernels.cuh): the tile layout chosen at
     // plan creation, or r == 0 when the plan streams its wavefield.
     struct Resident {
-        int r = 0, warps = 0;
+        int layout = -1;        // index into RES_LAYOUTS, -1: streaming
         bool surface = false;   // laid out with room for a topography mask
         int max_src = 0, max_rec_all = 0, max_rec = 0;  // point entries per tile: sources, receivers, owned receivers
         int4 *d_tiles = nullptr, *d_shot_tiles = nullptr;
         int *d_sync = nullptr;   // checks passed per shot
         uint4 *d_box = nullptr;  // outboxes of the largest launch
         size_t box_bytes = 0;
+        int box_stride = 0;
         unsigned tag = 0;        // tags used by the current call
         std::vector<int2> waves;  // (first tile, tiles) of each launch
         void *base = nullptr;     // their allocation
@@ -555,50 +556,62 @@ int read_status(rtm_plan *p, int32_t *flags, cudaStream_t s) {
 
 // ---- resident propagation (resident_kernels.cuh)
 
-// Tile layouts and the time of one step (us, mean of the two directions, 200 to
-// 600 steps of one source and a receiver on every row, measured) with 1, 2, ...
-// of their CTAs on every SM.  Few rows per lane finish a step soonest; many keep
-// more cells on the chip and recompute a smaller share of halo.  Layouts that
-// another one beats at every size are not built (P-SV R 4 x 8 warps: 432 CTAs
-// hold 581,000 cells at 3.7 us, R 6 x 8: 288 hold 645,000 at 3.3; R 3 x 16 is
-// 5 % behind R 6 x 8).
+// Tile layouts (rows per lane of the P-SV and of the SH tiles, warps) and the
+// time of one step (us, mean of the two directions, 200 to 600 steps of one
+// source and a receiver on every row, measured) with 1, 2, ... CTAs on every SM.
+// Few rows per lane finish a step soonest; many keep more cells on the chip and
+// recompute a smaller share of halo.  Layouts that another one beats at every
+// size are not built (P-SV R 4 x 8 warps: 432 CTAs hold 581,000 cells at 3.7 us,
+// R 6 x 8: 288 hold 645,000 at 3.3; R 3 x 16 is 5 % behind R 6 x 8; R 7 and 8
+// spill: 188 / 163 and 139 Gcell/s against 190).
 struct ResLayout {
-    int mode, r, warps;
+    int mode, rp, rs, warps;
     float us[4];
 };
 constexpr ResLayout RES_LAYOUTS[] = {
-    {RTM_PSV, 2, 8, {1.05f, 1.37f, 1.78f, 2.25f}}, {RTM_PSV, 2, 12, {1.31f, 1.90f}}, {RTM_PSV, 6, 8, {2.15f, 3.30f}},
-    {RTM_SH, 2, 8, {0.85f, 1.03f, 1.23f, 1.50f}},  {RTM_SH, 4, 8, {1.20f, 1.55f, 1.85f, 2.35f}}, {RTM_SH, 8, 8, {1.53f, 2.17f}},
-    {RTM_BOTH, 2, 8, {1.85f, 2.70f, 3.75f}},       {RTM_BOTH, 2, 16, {2.20f}},       {RTM_BOTH, 4, 8, {2.90f, 4.30f}},
+    {RTM_PSV, 2, 0, 8, {1.05f, 1.37f, 1.78f, 2.25f}}, {RTM_PSV, 2, 0, 12, {1.31f, 1.90f}}, {RTM_PSV, 6, 0, 8, {2.15f, 3.30f}},
+    {RTM_SH, 0, 2, 8, {0.85f, 1.03f, 1.23f, 1.50f}},  {RTM_SH, 0, 4, 8, {1.20f, 1.55f, 1.85f, 2.35f}}, {RTM_SH, 0, 8, 8, {1.53f, 2.17f}},
+    {RTM_BOTH, 2, 2, 8, {1.07f, 1.35f, 1.94f, 2.50f}}, {RTM_BOTH, 6, 8, 8, {2.27f, 3.15f}},
 };
-// Time of one step of the streaming kernels at their tuned shapes (us): small
-// grids are bound by the launch (one per two steps), large ones by issue.
-double streaming_us(int modes, long long cells) {
-    return 3.5 + (double)cells / (modes == RTM_PSV ? 170e3 : modes == RTM_SH ? 250e3 : 105e3);
+// Time of one step of the streaming kernels at their tuned shapes (us): the
+// launch (one per two steps), the last wave's tail, and the cells at the full
+// rate, strips of 120 columns counted whole.  Fits 0.47 to 28 million cells
+// within 10 %.
+double streaming_us(int modes, long long rows, int nz) {
+    const double cells = (double)rows * nz, padded = (double)rows * ((nz + 119) / 120 * 120);
+    const double tail = std::min(1.0, cells / 3e6);
+    if (modes == RTM_PSV) return 3.5 + 5.83e-6 * padded + 7.0 * tail;
+    if (modes == RTM_SH) return 3.5 + 3.7e-6 * padded + 3.5 * tail;
+    return 3.5 + 9.5e-6 * padded + 4.0 * tail;
 }
 
-// Calls f(dir, mode, R, NW) tags for a tile layout that exists; false else.
+// Calls f(kernel, P-SV layout, SH layout) for a tile layout; false if there is none.
 template <int DIR, typename F>
-bool res_dispatch(int mode, int r, int warps, F &&f) {
-#define RES_CASE(M, RR, NN)                                                                                  \
-    if (mode == M && r == RR && warps == NN) {                                                               \
-        f(std::integral_constant<int, DIR>{}, std::integral_constant<int, M>{}, std::integral_constant<int, RR>{}, \
-          std::integral_constant<int, NN>{});                                                                \
-        return true;                                                                                         \
+bool res_dispatch(const ResLayout &l, F &&f) {
+#define RES_ONE(M, RR, NN)                                                                             \
+    if (l.mode == M && (M == RTM_PSV ? l.rp : l.rs) == RR && l.warps == NN) {                           \
+        f((const void *)resident_kernel<DIR, M, RR, NN>, ResSmem<M, RR, NN>(), ResSmem<M, RR, NN>());   \
+        return true;                                                                                   \
     }
-    RES_CASE(RTM_PSV, 2, 8) RES_CASE(RTM_PSV, 2, 12) RES_CASE(RTM_PSV, 6, 8)
-    RES_CASE(RTM_SH, 2, 8) RES_CASE(RTM_SH, 4, 8) RES_CASE(RTM_SH, 8, 8)
-    RES_CASE(RTM_BOTH, 2, 8) RES_CASE(RTM_BOTH, 2, 16) RES_CASE(RTM_BOTH, 4, 8)
-#undef RES_CASE
+#define RES_TWO(RP, RS, NN)                                                                            \
+    if (l.mode == RTM_BOTH && l.rp == RP && l.rs == RS && l.warps == NN) {                              \
+        f((const void *)resident_both_kernel<DIR, RP, RS, NN>, ResSmem<1, RP, NN>(), ResSmem<2, RS, NN>()); \
+        return true;                                                                                   \
+    }
+    RES_ONE(RTM_PSV, 2, 8) RES_ONE(RTM_PSV, 2, 12) RES_ONE(RTM_PSV, 6, 8)
+    RES_ONE(RTM_SH, 2, 8) RES_ONE(RTM_SH, 4, 8) RES_ONE(RTM_SH, 8, 8)
+    RES_TWO(2, 2, 8) RES_TWO(6, 8, 8)
+#undef RES_ONE
+#undef RES_TWO
     return false;
 }
 
-size_t resident_smem(const rtm_plan *p, int r, int warps, int max_inj, int max_rec, bool surface, size_t *box = nullptr) {
+// Shared memory of a CTA and the packets of its two outboxes.
+size_t resident_smem(const ResLayout &l, int max_inj, int max_rec, bool surface, int *box = nullptr) {
     size_t n = 0;
-    res_dispatch<0>(p->g.modes, r, warps, [&](auto, auto m, auto rr, auto nn) {
-        using L = ResSmem<decltype(m)::value, decltype(rr)::value, decltype(nn)::value>;
-        n = L::bytes(surface, max_inj, max_rec);
-        if (box) *box = 2 * (size_t)L::BOX * sizeof(uint4);
+    res_dispatch<0>(l, [&](const void *, auto a, auto b) {
+        n = std::max(a.bytes(surface, max_inj, max_rec), b.bytes(surface, max_inj, max_rec));
+        if (box) *box = 2 * std::max(a.BOX, b.BOX);
     });
     return n;
 }
@@ -649,6 +662,7 @@ void resident_params(const rtm_plan *p, ResParams &rp, int dir) {
     rp.tiles = p->res.d_tiles;
     rp.shot_tiles = p->res.d_shot_tiles;
     rp.outbox = p->res.d_box;
+    rp.box_stride = p->res.box_stride;
     rp.arrive = p->res.d_sync;
     rp.max_inj = dir == 0 ? p->res.max_src : p->res.max_rec_all;
     rp.max_rec = dir == 0 ? p->res.max_rec : 0;
@@ -665,20 +679,18 @@ int resident_begin(rtm_plan *p, cudaStream_t s) {
 // Run the loop of rp for every shot, wave by wave.
 int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
     CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
+    const ResLayout &lay = RES_LAYOUTS[p->res.layout];
+    const size_t smem = resident_smem(lay, rp.max_inj, rp.max_rec, p->res.surface);
     const unsigned blocks = (unsigned)resident_blocks(rp.it0, rp.it1, rp.check_interval);
-    const size_t smem = resident_smem(p, p->res.r, p->res.warps, rp.max_inj, rp.max_rec, p->res.surface);
+    const void *kernel = nullptr;
+    auto take = [&](const void *k, auto, auto) { kernel = k; };
+    if (dir == 0) res_dispatch<0>(lay, take);
+    else res_dispatch<1>(lay, take);
     for (const int2 &w : p->res.waves) {
         rp.tile0 = w.x;
         rp.tag0 = p->res.tag;
-        cudaError_t e = cudaErrorInvalidValue;
-        auto go = [&](auto d, auto m, auto r, auto n) {
-            void *args[] = {&rp};
-            auto *k = resident_kernel<decltype(d)::value, decltype(m)::value, decltype(r)::value, decltype(n)::value>;
-            e = cudaLaunchCooperativeKernel((const void *)k, dim3(w.y), dim3(32 * p->res.warps), args, smem, s);
-        };
-        if (dir == 0) res_dispatch<0>(p->g.modes, p->res.r, p->res.warps, go);
-        else res_dispatch<1>(p->g.modes, p->res.r, p->res.warps, go);
-        CUDA_TRY(e);
+        void *args[] = {&rp};
+        CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(w.y), dim3(32 * lay.warps), args, smem, s));
         ++p->launches;
         p->res.tag += blocks;
     }
@@ -686,8 +698,8 @@ int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
 }
 
 // Choose the layout in which every shot's tiles are resident together and the
-// estimated step is shortest, and build its tables.  Leaves p->res.r at 0 when
-// there is none, or when streaming is estimated to be faster.
+// estimated step is shortest, and build its tables.  Leaves p->res.layout at -1
+// when there is none, or when streaming is estimated to be faster.
 int resident_setup(rtm_plan *p, bool surface) {
     const std::vector<int> &src_ptr = p->src_ptr_h, &rec_ptr = p->rec_ptr_h;
     const std::vector<int2> &src_ent = p->src_ent_h, &rec_ent = p->rec_ent_h;
@@ -703,46 +715,51 @@ int resident_setup(rtm_plan *p, bool surface) {
     const int ntz = (p->g.nz + ow - 1) / ow;
     rtm_plan::Resident best;
     std::vector<int4> tiles, stiles;
-    double best_us = streaming_us(p->g.modes, p->rows_total * p->g.nz);
-    for (const ResLayout &lay : RES_LAYOUTS) {
+    double best_us = streaming_us(p->g.modes, p->rows_total, p->g.nz);
+    for (int li = 0; li < (int)(sizeof RES_LAYOUTS / sizeof *RES_LAYOUTS); ++li) {
+        const ResLayout &lay = RES_LAYOUTS[li];
         if (lay.mode != p->g.modes) continue;
-        const int r = lay.r, warps = lay.warps, oh = warps * r - 2 * RES_HALO;
-        // tiles of every shot; point entries of the fullest tile
-        std::vector<int4> st;
+        // per wave type: rows a tile owns, tiles of every shot; point entries of the fullest tile
+        const int oh[2] = {lay.warps * lay.rp - 2 * RES_HALO, lay.warps * lay.rs - 2 * RES_HALO};
+        std::vector<int4> st((size_t)2 * p->nshots, make_int4(0, 0, ntz, 0));
         int max_src = 0, max_rec_all = 0, max_rec = 0, most = 0;
         for (int s = 0; s < p->nshots; ++s) {
             const ShotDev &d = p->shots_h[s];
-            const int ntx = (d.nx + oh - 1) / oh;
-            st.push_back(make_int4(0, ntx, ntz, 0));
-            most = std::max(most, ntx * ntz);
-            auto count = [&](const std::vector<int> &ptr, const std::vector<int2> &ent, int base, int ring) {
-                std::vector<int> n((size_t)ntx * ntz, 0);
-                for (int i = 0; i < d.nx; ++i)
-                    for (int e = ptr[base + i]; e < ptr[base + i + 1]; ++e)
-                        for (int a = std::max(0, (i - ring) / oh); a <= std::min(ntx - 1, (i + ring) / oh); ++a)
-                            for (int b = std::max(0, (ent[e].x - ring) / ow); b <= std::min(ntz - 1, (ent[e].x + ring) / ow); ++b)
-                                ++n[(size_t)a * ntz + b];
-                return *std::max_element(n.begin(), n.end());
-            };
-            max_src = std::max(max_src, count(src_ptr, src_ent, d.src_row0, RES_HALO));
-            max_rec_all = std::max(max_rec_all, count(rec_ptr, rec_ent, d.rec_row0, RES_HALO));
-            max_rec = std::max(max_rec, count(rec_ptr, rec_ent, d.rec_row0, 0));
+            for (int m = 0; m < 2; ++m) {
+                if (oh[m] <= 0) continue;
+                const int ntx = (d.nx + oh[m] - 1) / oh[m];
+                st[2 * s + m].y = ntx;
+                auto count = [&](const std::vector<int> &ptr, const std::vector<int2> &ent, int base, int ring) {
+                    std::vector<int> n((size_t)ntx * ntz, 0);
+                    for (int i = 0; i < d.nx; ++i)
+                        for (int e = ptr[base + i]; e < ptr[base + i + 1]; ++e)
+                            for (int a = std::max(0, (i - ring) / oh[m]); a <= std::min(ntx - 1, (i + ring) / oh[m]); ++a)
+                                for (int b = std::max(0, (ent[e].x - ring) / ow); b <= std::min(ntz - 1, (ent[e].x + ring) / ow); ++b)
+                                    ++n[(size_t)a * ntz + b];
+                    return *std::max_element(n.begin(), n.end());
+                };
+                max_src = std::max(max_src, count(src_ptr, src_ent, d.src_row0, RES_HALO));
+                max_rec_all = std::max(max_rec_all, count(rec_ptr, rec_ent, d.rec_row0, RES_HALO));
+                max_rec = std::max(max_rec, count(rec_ptr, rec_ent, d.rec_row0, 0));
+            }
+            const int n = (st[2 * s].y + st[2 * s + 1].y) * ntz;
+            st[2 * s].x = st[2 * s + 1].x = n;
+            most = std::max(most, n);
         }
         // CTAs per SM: the smaller of the two directions'
         int ctas = 0;
         cudaError_t e = cudaSuccess;
         for (int dir = 0; dir < 2; ++dir) {
-            const size_t smem = resident_smem(p, r, warps, dir == 0 ? max_src : max_rec_all, dir == 0 ? max_rec : 0, surface);
+            const size_t smem = resident_smem(lay, dir == 0 ? max_src : max_rec_all, dir == 0 ? max_rec : 0, surface);
             int c = 0;
-            auto query = [&](auto dd, auto m, auto rr, auto nn) {
-                auto *k = resident_kernel<decltype(dd)::value, decltype(m)::value, decltype(rr)::value, decltype(nn)::value>;
+            auto query = [&](const void *k, auto, auto) {
                 // the limit is the kernel's, not the plan's: always the largest
                 e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, 32 * warps, smem);
+                if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, 32 * lay.warps, smem);
             };
             if (smem <= 227 * 1024) {
-                if (dir == 0) res_dispatch<0>(p->g.modes, r, warps, query);
-                else res_dispatch<1>(p->g.modes, r, warps, query);
+                if (dir == 0) res_dispatch<0>(lay, query);
+                else res_dispatch<1>(lay, query);
             }
             if (e != cudaSuccess) c = 0;
             ctas = dir == 0 ? c : std::min(ctas, c);
@@ -753,21 +770,20 @@ int resident_setup(rtm_plan *p, bool surface) {
         const int capacity = ctas * sms;
         if (most > capacity || max_rec_all > RES_MAX_POINTS) continue;
         // launches: shots by decreasing tile count, each into the first one with room
-        auto ntiles = [&](int s) { return st[s].y * st[s].z; };
         std::vector<int> order(p->nshots);
         for (int s = 0; s < p->nshots; ++s) order[s] = s;
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ntiles(a) > ntiles(b); });
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return st[2 * a].x > st[2 * b].x; });
         std::vector<std::vector<int>> bins;
         std::vector<int> room;
         for (int s : order) {
             size_t b = 0;
-            while (b < bins.size() && room[b] < ntiles(s)) ++b;
+            while (b < bins.size() && room[b] < st[2 * s].x) ++b;
             if (b == bins.size()) {
                 bins.push_back({});
                 room.push_back(capacity);
             }
             bins[b].push_back(s);
-            room[b] -= ntiles(s);
+            room[b] -= st[2 * s].x;
         }
         double us = 0;
         for (int left : room) us += lay.us[(capacity - left + sms - 1) / sms - 1];
@@ -777,28 +793,27 @@ int resident_setup(rtm_plan *p, bool surface) {
         tiles.clear();
         for (auto &bin : bins) {
             const int t0 = (int)tiles.size();
-            for (int s : bin) {
-                st[s].x = (int)tiles.size();
-                for (int a = 0; a < st[s].y; ++a)
-                    for (int b = 0; b < ntz; ++b) tiles.push_back(make_int4(s, a * oh, b * ow, a * ntz + b));
-            }
+            for (int s : bin)
+                for (int m = 0; m < 2; ++m)
+                    for (int a = 0; a < st[2 * s + m].y; ++a)
+                        for (int b = 0; b < ntz; ++b) tiles.push_back(make_int4(s, a * oh[m], b * ow, m));
             best.waves.push_back(make_int2(t0, (int)tiles.size() - t0));
         }
         stiles = std::move(st);
-        best.r = r;
-        best.warps = warps;
+        best.layout = li;
         best.max_src = max_src;
         best.max_rec_all = max_rec_all;
         best.max_rec = max_rec;
     }
-    if (!best.r) return 0;
+    if (best.layout < 0) return 0;
     best.surface = surface;
     p->res = best;
-    size_t box = 0;
-    resident_smem(p, best.r, best.warps, 0, 0, false, &box);
+    int box = 0;
+    resident_smem(RES_LAYOUTS[best.layout], 0, 0, false, &box);
     int wide = 0;
     for (const int2 &w : best.waves) wide = std::max(wide, w.y);
-    p->res.box_bytes = box * wide;
+    p->res.box_stride = box;
+    p->res.box_bytes = (size_t)box * sizeof(uint4) * wide;
     Slab slab;
     slab.add(&p->res.d_tiles, tiles.size());
     slab.add(&p->res.d_shot_tiles, stiles.size());
@@ -1061,7 +1076,7 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     return RTM_OK;
 }
 
-int rtm_plan_resident(const rtm_plan *p) { return p && p->res.r > 0 ? 1 : 0; }
+int rtm_plan_resident(const rtm_plan *p) { return p && p->res.layout >= 0 ? 1 : 0; }
 
 int rtm_plan_destroy(rtm_plan *p) {
     if (!p) return RTM_OK;
@@ -1168,7 +1183,7 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
     if (save)
         for (float *b : {snap_u, snap_v, snap_w}) bs.add(b, rtm_plan_snapshot_floats(p, nsnap) * sizeof(float));
     if (int rc = bs.begin(s)) return rc;
-    const bool resident = p->res.r > 0 && !p->cb;
+    const bool resident = p->res.layout >= 0 && !p->cb;
     if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
     // Snapshot slots the time loop never reaches ((k+1)*isnap > nt-1) stay
     // zero, like the reference's zero-initialised fields (fm:533-535).
@@ -1308,7 +1323,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
     bs.add(stack, (size_t)3 * p->g.nx * p->g.nz * sizeof(double));
     if (int rc = bs.begin(s)) return rc;
     // the resident kernel images at every multiple of isnap that has a slot
-    bool resident = p->res.r > 0 && !p->cb;
+    bool resident = p->res.layout >= 0 && !p->cb;
     for (int k = 0; k < num_snaps; ++k)
         if ((long long)(k + 1) * isnap <= nt - 1 && isnaps[k] != (k + 1) * isnap) resident = false;
     if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
@@ -1612,7 +1627,7 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
     bs.add(seis, (size_t)3 * p->nrec_total * nt * sizeof(float));
     bs.add(ckpt, rtm_plan_checkpoint_bytes(p, ckpt_every, ckpt_dtype));
     if (int rc = bs.begin(s)) return rc;
-    const bool resident = p->res.r > 0;
+    const bool resident = p->res.layout >= 0;
     if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
     // every slot starts at zero: pad rows / columns of FP32 slots, and the
     // slots of a shot that stops before reaching them
@@ -1947,7 +1962,7 @@ int rtm_backward_checkpointed(rtm_plan *p, const float *wavelets, const float *o
     p->live = -1;
     auto body = [&]() -> int {
         if (int rc = bs.begin(s)) return rc;
-        const bool resident = p->res.r > 0;
+        const bool resident = p->res.layout >= 0;
         if (int rc = resident ? zero_status(p, s) : zero_state(p, s)) return rc;
         if (!resident) CUDA_TRY(cudaMemsetAsync(buf, 0, nbuf * sizeof(float), s));
         else if (int rc = resident_begin(p, s)) return rc;
