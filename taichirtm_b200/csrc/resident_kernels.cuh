@@ -58,6 +58,7 @@ struct ResParams {
     float *snap[3];
     int nsnap;                 // snapshot slots per shot in the buffers
     float *img[3], *imgc[3];
+    bool img_chip;             // backward: images kept in shared memory
     int *flags, *fail_seq;     // per shot: status, step + 1 of the first failed check
     int code_base;
     // loop: steps it0 .. it1-1; the time of step it is it (forward) or nt-1-it (backward)
@@ -110,6 +111,8 @@ struct ResSmem {
     static size_t bytes(bool surface, int max_inj, int max_rec) {
         return VAR + (size_t)max_inj * 8 + (size_t)max_rec * 8 + (size_t)RES_HALO * NC * max_inj * 4 + (surface ? CELLS * 8 : 0);
     }
+    // images on the chip: sum, compensation and the next snapshot of each component
+    static size_t image_bytes() { return (size_t)CELLS * NC * 3 * 8; }
 };
 
 // The point table says for each pair of cells which receiver entry it holds
@@ -199,6 +202,11 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     // this lane's cell of row 0; row r is 32 cells on
     const int cell0 = warp * (R * 32) + lane;
     unsigned char *const c16 = sm0 + cell0 * 16, *const c8 = sm0 + cell0 * 8;
+    // image rows (img_chip): [component][sum, compensation, snapshot][cell]
+    auto s_img = [&](int comp, int what, int r) -> f2 & {
+        f2 *b = s_sm() + (p.surface ? L::CELLS : 0);
+        return b[(size_t)(comp * 3 + what) * L::CELLS + cell0 + 32 * r];
+    };
     auto at16 = [&](int off, int r) { return *reinterpret_cast<const ulonglong2 *>(c16 + off + r * 512); };
     auto at8 = [&](int off, int r) { return *reinterpret_cast<const f2 *>(c8 + off + r * 256); };
     // this warp's published row of component comp; the warps above and below: -256, +256 bytes
@@ -672,6 +680,24 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             // per 500-step RTM.  Taller ones have no registers for it: the spills
             // cost every step (R 6: 3.0 -> 3.4 us).
             const long long io = (info->row_off + row0) * P + col + COL_OFF;
+            if (p.img_chip) {
+                cp_async_wait<0>();  // this lane's own copies of the snapshot
+                auto image = [&](int comp, int r, f2 v) {
+                    const f2 sn = s_img(comp, 2, r), im = s_img(comp, 0, r), ic = s_img(comp, 1, r);
+                    float s0 = f2_lo(im), c0 = f2_lo(ic), s1 = f2_hi(im), c1 = f2_hi(ic);
+                    kahan_add(s0, c0, __fmul_rn(f2_lo(sn), f2_lo(v)));
+                    kahan_add(s1, c1, __fmul_rn(f2_hi(sn), f2_hi(v)));
+                    s_img(comp, 0, r) = f2_pack(s0, s1);
+                    s_img(comp, 1, r) = f2_pack(c0, c1);
+                };
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (!(own >> r & 1)) continue;
+                    if constexpr (PSV) { image(0, r, U[r]); image(1, r, W[r]); }
+                    if constexpr (SH) image(CV, r, V[r]);
+                }
+                return;
+            }
             auto update = [&](int c, int r, f2 sn, f2 im, f2 ic, f2 v) {
                 float s0 = f2_lo(im), c0 = f2_lo(ic), s1 = f2_hi(im), c1 = f2_hi(ic);
                 kahan_add(s0, c0, __fmul_rn(f2_lo(sn), f2_lo(v)));
@@ -715,6 +741,42 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             }
         }
     };
+    // img_chip: copy snapshot slot k's pairs in (each lane its own, so its own
+    // wait is enough), and move the images in or out.
+    auto fetch_snapshot = [&](int k) {
+        const int row0 = my_row0(), col = my_col(), nx = info->nx;
+        const unsigned own = lane_owned(col) ? rows_own(row0, nx) : 0u;
+        const long long o = ((long long)p.nsnap * info->row_off + (long long)k * nx + row0) * p.pitch + col + COL_OFF;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!(own >> r & 1)) continue;
+            auto get = [&](int comp, int c) { cp_async_vec<2>(reinterpret_cast<float *>(&s_img(comp, 2, r)), p.snap[c] + o + (long long)r * p.pitch); };
+            if constexpr (PSV) { get(0, 0); get(1, 2); }
+            if constexpr (SH) get(CV, 1);
+        }
+        cp_async_commit();
+    };
+    auto move_images = [&](bool in) {
+        const int row0 = my_row0(), col = my_col();
+        const unsigned own = lane_owned(col) ? rows_own(row0, info->nx) : 0u;
+        const long long io = (info->row_off + row0) * (long long)p.pitch + col + COL_OFF;
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            if (!(own >> r & 1)) continue;
+            auto move = [&](int comp, int c) {
+                const long long at = io + (long long)r * p.pitch;
+                if (in) {
+                    s_img(comp, 0, r) = ld2(p.img[c], at);
+                    s_img(comp, 1, r) = ld2(p.imgc[c], at);
+                } else {
+                    st2(p.img[c], at, s_img(comp, 0, r));
+                    st2(p.imgc[c], at, s_img(comp, 1, r));
+                }
+            };
+            if constexpr (PSV) { move(0, 0); move(1, 2); }
+            if constexpr (SH) move(CV, 1);
+        }
+    };
     // Finite check (fm:455-488, bm:417-450) of the owned cells.
     auto check = [&](int seq) {
         int code = 0;
@@ -740,6 +802,11 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     publish_sig();
     int it = p.it0, checks = 0, blk = 0;
     int phase = p.isnap > 0 ? (DIR == 0 ? it : p.nt - 1 - it) % p.isnap : 1;  // t % isnap
+    if (DIR == 1 && p.img_chip) {
+        move_images(true);
+        const int m = min((p.nt - 1 - it) / p.isnap, p.snap_hi);  // the first imaging time is m * isnap
+        if (m >= p.snap_lo && m * p.isnap >= p.nt - p.it1) fetch_snapshot(m - p.snap_base);
+    }
     while (it < p.it1) {
         // steps of this block: up to H, ending at a checked step
         int n = min(RES_HALO, p.it1 - it);
@@ -915,7 +982,12 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             if constexpr (DIR == 0) { if (points) record(t); }
             if (phase == 0) {
                 const int m = t / p.isnap;
-                if (m >= p.snap_lo && m <= p.snap_hi) snapshot(m - p.snap_base);
+                if (m >= p.snap_lo && m <= p.snap_hi) {
+                    snapshot(m - p.snap_base);
+                    // the next one's copies are under way while the steps up to it run
+                    if (DIR == 1 && p.img_chip && m - 1 >= p.snap_lo && (m - 1) * p.isnap >= p.nt - p.it1)
+                        fetch_snapshot(m - 1 - p.snap_base);
+                }
             }
             if (p.isnap > 0) {
                 if constexpr (DIR == 0) phase = phase + 1 == p.isnap ? 0 : phase + 1;
@@ -940,6 +1012,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         }
     }
     cp_async_wait<0>();
+    if (DIR == 1 && p.img_chip) move_images(false);
     // final state of the owned cells; a shot that stopped inside a segment leaves none
     if (p.store[PSV ? F_U : F_V] && !(p.segment && info->leave == 2 && it < p.it1)) {
         const int row0 = my_row0(), col = my_col();

@@ -165,6 +165,7 @@ struct rtm_plan {
         size_t box_bytes = 0;
         int box_stride = 0;
         unsigned tag = 0;        // tags used by the current call
+        bool image_fits = false; // every launch fits with its images in shared memory
         std::vector<int2> waves;  // (first tile, tiles) of each launch
         void *base = nullptr;     // their allocation
     } res;
@@ -607,9 +608,10 @@ bool res_dispatch(const ResLayout &l, F &&f) {
 }
 
 // Shared memory of a CTA and the packets of its two outboxes.
-size_t resident_smem(const ResLayout &l, int max_inj, int max_rec, bool surface, int *box = nullptr) {
+size_t resident_smem(const ResLayout &l, int max_inj, int max_rec, bool surface, int *box = nullptr, size_t *image = nullptr) {
     size_t n = 0;
     res_dispatch<0>(l, [&](const void *, auto a, auto b) {
+        if (image) *image = std::max(a.image_bytes(), b.image_bytes());
         n = std::max(a.bytes(surface, max_inj, max_rec), b.bytes(surface, max_inj, max_rec));
         if (box) *box = 2 * std::max(a.BOX, b.BOX);
     });
@@ -680,7 +682,10 @@ int resident_begin(rtm_plan *p, cudaStream_t s) {
 int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
     CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
     const ResLayout &lay = RES_LAYOUTS[p->res.layout];
-    const size_t smem = resident_smem(lay, rp.max_inj, rp.max_rec, p->res.surface);
+    size_t image = 0, smem = resident_smem(lay, rp.max_inj, rp.max_rec, p->res.surface, nullptr, &image);
+    // images stay on the chip where every launch still fits with them
+    rp.img_chip = dir == 1 && rp.isnap > 0 && p->res.image_fits;
+    if (rp.img_chip) smem += image;
     const unsigned blocks = (unsigned)resident_blocks(rp.it0, rp.it1, rp.check_interval);
     const void *kernel = nullptr;
     auto take = [&](const void *k, auto, auto) { kernel = k; };
@@ -746,11 +751,13 @@ int resident_setup(rtm_plan *p, bool surface) {
             st[2 * s].x = st[2 * s + 1].x = n;
             most = std::max(most, n);
         }
-        // CTAs per SM: the smaller of the two directions'
-        int ctas = 0;
+        // CTAs per SM: the smaller of the two directions'; and backward with images
+        int ctas = 0, ctas_image = 0;
         cudaError_t e = cudaSuccess;
-        for (int dir = 0; dir < 2; ++dir) {
-            const size_t smem = resident_smem(lay, dir == 0 ? max_src : max_rec_all, dir == 0 ? max_rec : 0, surface);
+        for (int pass = 0; pass < 3; ++pass) {
+            const int dir = std::min(pass, 1);
+            size_t image = 0, smem = resident_smem(lay, dir == 0 ? max_src : max_rec_all, dir == 0 ? max_rec : 0, surface, nullptr, &image);
+            if (pass == 2) smem += image;
             int c = 0;
             auto query = [&](const void *k, auto, auto) {
                 // the limit is the kernel's, not the plan's: always the largest
@@ -762,7 +769,7 @@ int resident_setup(rtm_plan *p, bool surface) {
                 else res_dispatch<1>(lay, query);
             }
             if (e != cudaSuccess) c = 0;
-            ctas = dir == 0 ? c : std::min(ctas, c);
+            (pass == 2 ? ctas_image : ctas) = pass == 1 ? std::min(ctas, c) : c;
         }
         if (e != cudaSuccess) cudaGetLastError();
         ctas = std::min(ctas, 4);
@@ -800,6 +807,8 @@ int resident_setup(rtm_plan *p, bool surface) {
             best.waves.push_back(make_int2(t0, (int)tiles.size() - t0));
         }
         stiles = std::move(st);
+        best.image_fits = true;
+        for (const int2 &w : best.waves) best.image_fits = best.image_fits && w.y <= ctas_image * sms;
         best.layout = li;
         best.max_src = max_src;
         best.max_rec_all = max_rec_all;

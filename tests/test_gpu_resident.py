@@ -161,3 +161,38 @@ def test_checkpointed_segments(store, every, nt, isnap, check):
         p.close()
     assert np.abs(res[0][3]).max() > 0 and np.abs(res[0][4]).max() > 0
     _same(*res)
+
+
+def test_two_threads_and_streams():
+    """Two plans propagate at the same time, each in a host thread and on a
+    stream of its own; together they ask for more tiles than the chip holds."""
+    import threading
+    from taichirtm_b200.plan import Plan, ShotGeometry
+    nx, nz, nt = 300, 400, 200
+    src, rec = _points(nx, nz, dense=False)
+    wav = torch.as_tensor(_wavelets(len(src), nt)).cuda()
+    plans = []
+    for _ in range(2):
+        p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 20, 1, [ShotGeometry(0, nx, src, rec)])
+        p.set_model(*_model(nx, nz))
+        assert p.resident()
+        plans.append(p)
+    want = plans[0].forward(wav)[1].clone()
+    torch.cuda.synchronize()
+    same, errors = [], []
+
+    def work(p, stream):
+        try:
+            for _ in range(10):
+                flags, seis, _, _ = p.forward(wav, stream=stream)  # returns after the stream's work
+                same.append(flags[0] == 0 and torch.equal(seis, want))
+        except Exception as e:  # noqa: BLE001 - reported below
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(p, torch.cuda.Stream())) for p in plans]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    for p in plans:
+        p.close()
+    assert not errors and len(same) == 20 and all(same)
