@@ -68,6 +68,10 @@ struct ResParams {
     // state: loaded from load[] (null: zero), owned cells stored to store[] at the end (null: not)
     const float *load[NFIELD];
     float *store[NFIELD];
+    // forward, keep_every > 0: the state after every keep_every'th step of the launch
+    // before nt is stored instead, the first to store[], the next keep floats on, ...
+    int keep_every;
+    long long keep;
     // tiles
     const int4 *tiles;         // (shot, first owned row, first owned column, wave type); a shot's tiles row by row
     const int4 *shot_tiles;    // per shot, P-SV and SH: (tiles of the shot, tile rows, tile columns, unused)
@@ -798,6 +802,19 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         }
     };
 
+    // the state of the owned cells to store[] + at
+    auto store_state = [&](long long at) {
+        const int row0 = my_row0(), col = my_col();
+        if (!lane_owned(col)) return;
+        const unsigned own = rows_own(row0, info->nx);
+        const long long so = state_at(row0, col) + at;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (!(own >> r & 1)) continue;
+            store_row(r, so + (long long)r * p.pitch, p.store);
+        }
+    };
+
     // ---- time loop
     publish_sig();
     int it = p.it0, checks = 0, blk = 0;
@@ -979,7 +996,11 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             else stress(std::integral_constant<int, 3>{});
             publish_sig();
             const int t = DIR == 0 ? it : p.nt - 1 - it;
-            if constexpr (DIR == 0) { if (points) record(t); }
+            if constexpr (DIR == 0) {
+                if (points) record(t);
+                if (p.keep_every && (it + 1 - p.it0) % p.keep_every == 0 && it + 1 < p.nt)
+                    store_state(((it + 1 - p.it0) / p.keep_every - 1) * p.keep);
+            }
             if (phase == 0) {
                 const int m = t / p.isnap;
                 if (m >= p.snap_lo && m <= p.snap_hi) {
@@ -1014,17 +1035,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     cp_async_wait<0>();
     if (DIR == 1 && p.img_chip) move_images(false);
     // final state of the owned cells; a shot that stopped inside a segment leaves none
-    if (p.store[PSV ? F_U : F_V] && !(p.segment && info->leave == 2 && it < p.it1)) {
-        const int row0 = my_row0(), col = my_col();
-        if (!lane_owned(col)) return;
-        const unsigned own = rows_own(row0, info->nx);
-        const long long so = state_at(row0, col);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (!(own >> r & 1)) continue;
-            store_row(r, so + (long long)r * p.pitch, p.store);
-        }
-    }
+    if (p.store[PSV ? F_U : F_V] && !(DIR == 0 && p.keep_every) && !(p.segment && info->leave == 2 && it < p.it1)) store_state(0);
 }
 
 template <int DIR, int MODE, int R, int NW>

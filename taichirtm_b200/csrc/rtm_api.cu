@@ -680,7 +680,7 @@ int resident_begin(rtm_plan *p, cudaStream_t s) {
 
 // Run the loop of rp for every shot, wave by wave.
 int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
-    CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
+    if (rp.check_interval > 0) CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
     const ResLayout &lay = RES_LAYOUTS[p->res.layout];
     size_t image = 0, smem = resident_smem(lay, rp.max_inj, rp.max_rec, p->res.surface, nullptr, &image);
     // images stay on the chip where every launch still fits with them
@@ -1658,8 +1658,10 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
     auto check_at = [&](int it) { return check_interval > 0 && it % check_interval == 0; };
     auto save_at = [&](int it) { return (it + 1) % ckpt_every == 0 && it + 1 < nt; };
     if (resident) {
-        // one segment between checkpoints at a time, its end state stored in FP32:
-        // straight into an FP32 slot, or into a state buffer and packed from there
+        // FP32 slots are written by one launch over all steps.  16-bit ones are packed
+        // from a state buffer, one segment between checkpoints at a time.
+        const bool f32 = ckpt_dtype == RTM_CKPT_F32;
+        const int len = f32 ? nt : ckpt_every;
         ResParams rp;
         resident_params(p, rp, 0);
         for (int c = 0; c < 3; ++c) {
@@ -1668,20 +1670,22 @@ int rtm_forward_checkpointed(rtm_plan *p, const float *wavelets, float *seis, in
         }
         rp.code_base = 1;
         rp.check_interval = check_interval;
-        rp.segment = true;
+        rp.segment = !f32;
+        rp.keep_every = f32 ? ckpt_every : 0;
+        rp.keep = (long long)NADJ * p->state_floats;
         if (int rc = resident_begin(p, s)) return rc;
-        for (int start = 0, seg = 0; start < nt; start += ckpt_every, ++seg) {
-            const int end = std::min(start + ckpt_every, nt);
-            const bool save = end < nt, f32 = ckpt_dtype == RTM_CKPT_F32;
+        for (int start = 0, seg = 0; start < nt; start += len, ++seg) {
+            const int end = std::min(start + len, nt);
+            const bool save = !f32 && end < nt;
             float *dst[NADJ];
-            for (int f = 0; f < NADJ; ++f)
-                dst[f] = save && f32 ? reinterpret_cast<float *>(ckpt_slot(p, ckpt, ckpt_dtype, seg)) + (size_t)f * p->state_floats
-                                     : p->d_state[seg & 1][f];
-            for (int f = 0; f < NADJ; ++f) rp.store[f] = save ? dst[f] : nullptr;
+            for (int f = 0; f < NADJ; ++f) {
+                dst[f] = f32 && ckpt ? static_cast<float *>(ckpt) + (size_t)f * p->state_floats : p->d_state[seg & 1][f];
+                rp.store[f] = save || f32 ? dst[f] : nullptr;
+            }
             rp.it0 = start;
             rp.it1 = end;
             if (int rc = resident_run(p, rp, 0, s)) return rc;
-            if (save && !f32) {
+            if (save) {
                 if (int rc = ckpt_store(p, ckpt, ckpt_dtype, seg, dst, end, s)) return rc;
             }
             for (int f = 0; f < NADJ; ++f) rp.load[f] = dst[f];
@@ -1771,8 +1775,7 @@ int rtm_adjoint(rtm_plan *p, const float *wavelets, const float *resid, int ckpt
     p->live = -1;
     auto body = [&]() -> int {
         if (int r = bs.begin(s)) return r;
-        CUDA_TRY(cudaMemsetAsync(p->d_flags, 0, p->nshots * sizeof(int), s));
-        CUDA_TRY(cudaMemsetAsync(p->d_fail_seq, 0x7f, p->nshots * sizeof(int), s));
+        if (int r = zero_status(p, s)) return r;
         CUDA_TRY(cudaMemsetAsync(seg, 0, nslots * slot * sizeof(float), s));
         CUDA_TRY(cudaMemsetAsync(gsum, 0, (size_t)3 * NGRAD * gfl * sizeof(float), s));
         if (gwt) CUDA_TRY(cudaMemsetAsync(gwt, 0, (size_t)3 * nt * p->nsrc_total * sizeof(float), s));
@@ -1835,6 +1838,19 @@ int rtm_adjoint(rtm_plan *p, const float *wavelets, const float *resid, int ckpt
             fold.part[g] = gsum + (size_t)(2 * NGRAD + g) * gfl;
             ap.gpart[g] = fold.part[g];
         }
+        // A resident plan recomputes on the chip: 201 x 101, 300 steps, 1.? ms
+        const bool resident = p->res.layout >= 0;
+        ResParams rp;
+        if (resident) {
+            resident_params(p, rp, 0);
+            for (int c = 0; c < 3; ++c) {
+                rp.wav[c] = sp.wav[c];
+                rp.seis[c] = sp.seis[c];
+            }
+            rp.keep_every = 1;
+            rp.keep = (long long)slot;
+            if (int r = resident_begin(p, s)) return r;
+        }
         int cur = 0;
         const int warps = p->warps;
         const int blocks = (p->n_work + warps - 1) / warps;
@@ -1843,9 +1859,19 @@ int rtm_adjoint(rtm_plan *p, const float *wavelets, const float *resid, int ckpt
             const int start = sgi * K, end = std::min(start + K, nt);
             float *s0 = nullptr;
             if (int r = segment_start(p, ckpt, ckpt_dtype, sgi, zero, stage, &s0, s)) return r;
-            // recompute forward states start .. end-2 into seg slots 0 .. len-2,
-            // two steps per launch (each state stored) where the plan runs two
-            for (int it = start; it <= end - 2;) {
+            // recompute forward states start .. end-2 into seg slots 0 .. len-2: in one
+            // resident launch that stores the state of every step, or two steps
+            // per launch (each state stored) where the plan runs two
+            if (resident && end - start >= 2) {
+                for (int f = 0; f < NADJ; ++f) {
+                    rp.load[f] = fld(s0, f);
+                    rp.store[f] = fld(seg, f);
+                }
+                rp.it0 = start;
+                rp.it1 = end - 1;
+                if (int r = resident_run(p, rp, 0, s)) return r;
+            }
+            for (int it = start; !resident && it <= end - 2;) {
                 float *src = it == start ? s0 : seg + (size_t)(it - 1 - start) * slot;
                 float *dst = seg + (size_t)(it - start) * slot;
                 const bool two = p->tsteps == 2 && p->vec >= 2 && it + 1 <= end - 2;
@@ -1927,7 +1953,8 @@ int rtm_adjoint(rtm_plan *p, const float *wavelets, const float *resid, int ckpt
         if (gwt) {
             if (int r = transpose(gwt, grad_wavelet, 3, nt, p->nsrc_total, s)) return r;
         }
-        CUDA_TRY(cudaStreamSynchronize(s));
+        std::vector<int> status(p->nshots);
+        if (int r = read_status(p, status.data(), s)) return r;
         if (int r = bs.end(s)) return r;
         return RTM_OK;
     };
