@@ -79,7 +79,7 @@ struct ResParams {
     uint4 *outbox;             // per CTA of the launch: box_stride packets, two outboxes of ResSmem::BOX
     int box_stride;
     unsigned tag0;             // exchange b of this launch is tagged tag0 + b
-    int *arrive;               // per shot: checks passed, summed over its tiles
+    unsigned long long *arrive;  // per shot, odd and even checks: tiles that made it | tiles that failed it << 32
     int *err;
     int max_inj, max_rec;      // point entries a tile may hold (host-checked)
 };
@@ -131,7 +131,8 @@ struct ResInfo {
     int nx, shot, row0, col0;  // first owned row and column
     int nti, ntj;              // the shot's tile rows and columns
     int tiles;                 // tiles of the shot, of both wave types
-    int leave;
+    int leave;                 // 1: a wait ran out, 2: the shot failed its check
+    int bad;                   // this tile failed its check
 };
 static_assert(sizeof(ResInfo) <= 64, "");
 
@@ -164,14 +165,10 @@ __device__ __forceinline__ void st_if(float *p, float x, bool pred) {
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q st.global.f32 [%0], %1; }" ::"l"(p), "f"(x), "r"((unsigned)pred) : "memory");
 }
 
-// Wait until *p >= want (bounded; also gives up when *err is raised).
-__device__ __forceinline__ bool res_wait(const int *p, int want, int *err) {
-    for (int n = 0; n < RES_SPIN_LIMIT; ++n) {
-        if (ld_acquire(p) >= want) return true;
-        if ((n & 1023) == 1023 && ld_acquire(err) != 0) return false;
-    }
-    atomicExch(err, 1);
-    return false;
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 
 // CTAs per SM that the register budget is cut for: the wavefield takes 2 R
@@ -245,7 +242,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             info->nti = st.y;
             info->ntj = st.z;
             info->tiles = st.x;
-            info->leave = 0;
+            info->leave = info->bad = 0;
         }
         cm0 = (unsigned)(col - 1) < (unsigned)(nz - 2) ? ~0u : 0u;
         cm1 = (unsigned)col < (unsigned)(nz - 2) ? ~0u : 0u;
@@ -799,6 +796,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         if (lane == 0 && code > 0) {
             atomicMax(p.flags + info->shot, code);
             atomicMin(p.fail_seq + info->shot, seq);
+            info->bad = 1;
         }
     };
 
@@ -818,6 +816,12 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     // ---- time loop
     publish_sig();
     int it = p.it0, checks = 0, blk = 0;
+    bool check_last = false;  // the block before ended at a checked step
+    int next_check = p.it1;   // next checked step, p.it1: none left
+    if (p.check_interval > 0) {
+        const int d = it % p.check_interval;
+        next_check = d == 0 ? it : p.check_interval - d < p.it1 - it ? it + p.check_interval - d : p.it1;
+    }
     int phase = p.isnap > 0 ? (DIR == 0 ? it : p.nt - 1 - it) % p.isnap : 1;  // t % isnap
     if (DIR == 1 && p.img_chip) {
         move_images(true);
@@ -827,11 +831,8 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     while (it < p.it1) {
         // steps of this block: up to H, ending at a checked step
         int n = min(RES_HALO, p.it1 - it);
-        bool check_last = false;
-        if (p.check_interval > 0) {
-            const int d = (p.check_interval - it % p.check_interval) % p.check_interval + 1;
-            if (d <= n) { n = d; check_last = true; }
-        }
+        const bool made = check_last;
+        n = min(n, next_check - it + 1);
         // injection values of the block
         const int n_inj = s_ip[RT];
         for (int k = threadIdx.x; k < n * n_inj; k += 32 * NW) {
@@ -921,14 +922,28 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             // All packets are asked for at once, those still missing again together.
             // (Polling with three lanes first, to spare L2 the traffic, was slower:
             // 9,058 against 8,517 cycles per block on a 301 x 151 shot.)
+            // A check that the last block made is settled here too: every tile of the
+            // shot has sent its count by now, and nothing has been put out since.  (A
+            // wait of its own after the check took 6,000 cycles, most of them for the
+            // fence and the chain of three L2 round trips.)  Checks alternate between
+            // two counters, so a tile that is already past the next check cannot be
+            // mistaken for one that has made this one.
+            bool ask = made && threadIdx.x == 0;
+            const unsigned long long *const arrive = p.arrive + 2 * info->shot + (checks & 1);
             for (int n = 0;;) {
+                unsigned long long seen = 0;
+                if (ask) seen = ld_relaxed(arrive);
 #pragma unroll
                 for (int k = 0; k < FP + SP; ++k)
                     if (pending >> k & 1) ld_packet(pk[k], src[k]);
+                if (ask && (unsigned)seen == (unsigned)((checks + 1) / 2 * info->tiles)) {
+                    ask = false;
+                    if (seen >> 32) info->leave = 2;
+                }
 #pragma unroll
                 for (int k = 0; k < FP + SP; ++k)
                     if (pk[k].tag() == tag) pending &= ~(1u << k);
-                if (!pending) break;
+                if (!pending && !ask) break;
                 if (++n >= RES_SPIN_LIMIT || ((n & 1023) == 1023 && ld_acquire(p.err) != 0)) {
                     atomicExch(p.err, 1);
                     info->leave = 1;
@@ -1014,22 +1029,16 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 if constexpr (DIR == 0) phase = phase + 1 == p.isnap ? 0 : phase + 1;
                 else phase = phase == 0 ? p.isnap - 1 : phase - 1;
             }
-            if (check_last && s == n - 1) check(it + 1);
+            if (it == next_check) check(it + 1);
             __syncthreads();
         }
         ++blk;
+        check_last = it == next_check + 1;
         if (check_last) {
-            // every tile of the shot passes this check before any goes on
             ++checks;
-            if (threadIdx.x == 0) {
-                int *const arrive = p.arrive + info->shot;
-                __threadfence();
-                atomicAdd(arrive, 1);
-                if (!res_wait(arrive, checks * info->tiles, p.err)) info->leave = 1;
-                if (ld_acquire(p.fail_seq + info->shot) <= it) info->leave = 2;  // failed at this check
-            }
-            __syncthreads();
-            if (info->leave) break;
+            if (threadIdx.x == 0)
+                atomicAdd(p.arrive + 2 * info->shot + (checks & 1), info->bad ? (1ull << 32) + 1 : 1ull);
+            next_check = p.check_interval < p.it1 - next_check ? next_check + p.check_interval : p.it1;
         }
     }
     cp_async_wait<0>();

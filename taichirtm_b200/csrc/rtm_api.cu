@@ -160,7 +160,7 @@ struct rtm_plan {
         bool surface = false;   // laid out with room for a topography mask
         int max_src = 0, max_rec_all = 0, max_rec = 0;  // point entries per tile: sources, receivers, owned receivers
         int4 *d_tiles = nullptr, *d_shot_tiles = nullptr;
-        int *d_sync = nullptr;   // checks passed per shot
+        unsigned long long *d_sync = nullptr;  // per shot: ResParams::arrive
         uint4 *d_box = nullptr;  // outboxes of the largest launch
         size_t box_bytes = 0;
         int box_stride = 0;
@@ -680,7 +680,7 @@ int resident_begin(rtm_plan *p, cudaStream_t s) {
 
 // Run the loop of rp for every shot, wave by wave.
 int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
-    if (rp.check_interval > 0) CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, p->nshots * sizeof(int), s));
+    if (rp.check_interval > 0) CUDA_TRY(cudaMemsetAsync(p->res.d_sync, 0, 2 * p->nshots * sizeof(*p->res.d_sync), s));
     const ResLayout &lay = RES_LAYOUTS[p->res.layout];
     size_t image = 0, smem = resident_smem(lay, rp.max_inj, rp.max_rec, p->res.surface, nullptr, &image);
     // images stay on the chip where every launch still fits with them
@@ -826,7 +826,7 @@ int resident_setup(rtm_plan *p, bool surface) {
     Slab slab;
     slab.add(&p->res.d_tiles, tiles.size());
     slab.add(&p->res.d_shot_tiles, stiles.size());
-    slab.add(&p->res.d_sync, (size_t)p->nshots);
+    slab.add(&p->res.d_sync, 2 * (size_t)p->nshots);
     slab.add(&p->res.d_box, p->res.box_bytes / sizeof(uint4));
     if (int rc = slab.commit()) {
         p->res = rtm_plan::Resident();
