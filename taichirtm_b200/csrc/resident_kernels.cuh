@@ -108,7 +108,7 @@ struct ResSmem {
     static constexpr int BOX = ORW * OLN * NP;
     static constexpr int STAGE = (2 * RES_HALO * 32 + ORW * RES_HALO) * NF * 4, ROWBUF = 2 * (NW + 2) * 32 * 8 * NC;
     static constexpr int INFO = VEL + ((STAGE > ROWBUF ? STAGE : ROWBUF) + 15) / 16 * 16;  // ResInfo
-    static constexpr int PT = INFO + 64;                             // point table: 16 bits per (row, lane)
+    static constexpr int PT = INFO + 80;                             // point table: 16 bits per (row, lane)
     static constexpr int IP = PT + ROWS * 32 * 2;                    // row offsets of the entries
     static constexpr int RP = IP + (ROWS + 2) * 4;
     static constexpr int VAR = (RP + (ROWS + 2) * 4 + 15) / 16 * 16;
@@ -127,14 +127,15 @@ constexpr int RES_MAX_POINTS = 0x7ff0;  // receiver entries a tile may hold
 // What the exchange and the output rows need of a tile, kept in shared memory
 // so that it does not occupy registers between them.
 struct ResInfo {
-    long long state_off, row_off;
+    long long state_off, snap_off, img_off;  // of a shot's state; of tile cell (0, 0) in snapshot slot 0 and in the images
+    int slot;                  // floats of a snapshot slot
     int nx, shot, row0, col0;  // first owned row and column
     int nti, ntj;              // the shot's tile rows and columns
     int tiles;                 // tiles of the shot, of both wave types
     int leave;                 // 1: a wait ran out, 2: the shot failed its check
     int bad;                   // this tile failed its check
 };
-static_assert(sizeof(ResInfo) <= 64, "");
+static_assert(sizeof(ResInfo) <= 80, "");
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
     int v;
@@ -234,7 +235,10 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         if (p.segment && ld_acquire(p.fail_seq + tl.x) <= p.it0) return;
         if (threadIdx.x == 0) {
             info->state_off = sh.state_off;
-            info->row_off = sh.row_off;
+            const long long at = (long long)(tl.y - H) * P + (tl.z - H) + COL_OFF;
+            info->snap_off = (long long)p.nsnap * sh.row_off * P + at;
+            info->img_off = sh.row_off * P + at;
+            info->slot = nx * P;
             info->nx = nx;
             info->shot = tl.x;
             info->row0 = tl.y;
@@ -402,16 +406,16 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         for (int r = 0; r < R; ++r) m |= (unsigned)((unsigned)(row0 + r) < (unsigned)nx) << r;
         return m;
     };
-    auto rows_own = [&](int row0, int nx) {
-        unsigned m = 0;
+    // bit r: this lane's pair of row r is the tile's own, inside the window
+    unsigned own = 0;
+    if (lane >= RES_HALO / 2 && lane < 32 - RES_HALO / 2 && my_col() < p.nz) {
+        const int row0 = my_row0(), nx = info->nx;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int rr = warp * R + r;
-            m |= (unsigned)(rr >= RES_HALO && rr < RT - RES_HALO && row0 + r < nx) << r;
+            own |= (unsigned)(rr >= RES_HALO && rr < RT - RES_HALO && row0 + r < nx) << r;
         }
-        return m;
-    };
-    auto lane_owned = [&](int col) { return lane >= RES_HALO / 2 && lane < 32 - RES_HALO / 2 && col < p.nz; };
+    }
     auto state_at = [&](int row0, int col) { return info->state_off + (long long)(row0 + 1) * p.pitch + (col + COL_OFF); };
     {
         const int row0 = my_row0(), col = my_col(), nx = info->nx;
@@ -662,11 +666,10 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     };
     // Snapshot slot k (fm:490-497) or its correlation (bm:481-488), owned cells.
     auto snapshot = [&](int k) {
-        const int row0 = my_row0(), col = my_col(), nx = info->nx;
-        if (!lane_owned(col)) return;
-        const unsigned own = rows_own(row0, nx);
+        if (!own) return;
         const long long P = p.pitch;
-        const long long o = ((long long)p.nsnap * info->row_off + (long long)k * nx + row0) * P + col + COL_OFF;
+        const int cell = warp * R * p.pitch + 2 * lane;
+        const long long o = info->snap_off + (long long)k * info->slot + cell;
         if constexpr (DIR == 0) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -680,7 +683,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             // moved over the stores); 301 x 151, an image at every step: 2.70 -> 2.40 ms
             // per 500-step RTM.  Taller ones have no registers for it: the spills
             // cost every step (R 6: 3.0 -> 3.4 us).
-            const long long io = (info->row_off + row0) * P + col + COL_OFF;
+            const long long io = info->img_off + cell;
             if (p.img_chip) {
                 cp_async_wait<0>();  // this lane's own copies of the snapshot
                 auto image = [&](int comp, int r, f2 v) {
@@ -745,9 +748,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     // img_chip: copy snapshot slot k's pairs in (each lane its own, so its own
     // wait is enough), and move the images in or out.
     auto fetch_snapshot = [&](int k) {
-        const int row0 = my_row0(), col = my_col(), nx = info->nx;
-        const unsigned own = lane_owned(col) ? rows_own(row0, nx) : 0u;
-        const long long o = ((long long)p.nsnap * info->row_off + (long long)k * nx + row0) * p.pitch + col + COL_OFF;
+        const long long o = info->snap_off + (long long)k * info->slot + (warp * R * p.pitch + 2 * lane);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!(own >> r & 1)) continue;
@@ -758,9 +759,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         cp_async_commit();
     };
     auto move_images = [&](bool in) {
-        const int row0 = my_row0(), col = my_col();
-        const unsigned own = lane_owned(col) ? rows_own(row0, info->nx) : 0u;
-        const long long io = (info->row_off + row0) * (long long)p.pitch + col + COL_OFF;
+        const long long io = info->img_off + (warp * R * p.pitch + 2 * lane);
 #pragma unroll 1
         for (int r = 0; r < R; ++r) {
             if (!(own >> r & 1)) continue;
@@ -781,16 +780,12 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     // Finite check (fm:455-488, bm:417-450) of the owned cells.
     auto check = [&](int seq) {
         int code = 0;
-        const int row0 = my_row0(), col = my_col();
-        if (lane_owned(col)) {
-            const unsigned own = rows_own(row0, info->nx);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (!(own >> r & 1)) continue;
-                auto bad = [&](f2 x, int c) { code = max(code, max(bad_code(f2_lo(x), c), bad_code(f2_hi(x), c))); };
-                if constexpr (PSV) { bad(U[r], p.code_base); bad(W[r], p.code_base + 2); }
-                if constexpr (SH) bad(V[r], p.code_base + 1);
-            }
+        for (int r = 0; r < R; ++r) {
+            if (!(own >> r & 1)) continue;
+            auto bad = [&](f2 x, int c) { code = max(code, max(bad_code(f2_lo(x), c), bad_code(f2_hi(x), c))); };
+            if constexpr (PSV) { bad(U[r], p.code_base); bad(W[r], p.code_base + 2); }
+            if constexpr (SH) bad(V[r], p.code_base + 1);
         }
         code = __reduce_max_sync(FULL, code);
         if (lane == 0 && code > 0) {
@@ -802,10 +797,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
 
     // the state of the owned cells to store[] + at
     auto store_state = [&](long long at) {
-        const int row0 = my_row0(), col = my_col();
-        if (!lane_owned(col)) return;
-        const unsigned own = rows_own(row0, info->nx);
-        const long long so = state_at(row0, col) + at;
+        const long long so = state_at(my_row0(), my_col()) + at;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!(own >> r & 1)) continue;
@@ -822,11 +814,22 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         const int d = it % p.check_interval;
         next_check = d == 0 ? it : p.check_interval - d < p.it1 - it ? it + p.check_interval - d : p.it1;
     }
-    int phase = p.isnap > 0 ? (DIR == 0 ? it : p.nt - 1 - it) % p.isnap : 1;  // t % isnap
+    // the next imaging step and its m; p.it1 or later: none left.  (Found by a division
+    // per step, with the slot's offset from the window's: 500 cycles per step, on warps
+    // without a cell to store too.)
+    int img_it = p.it1, img_m = 0;
+    if (p.isnap > 0) {
+        if constexpr (DIR == 0) {
+            img_m = max(p.snap_lo, it / p.isnap + (it % p.isnap != 0));
+            if (img_m <= p.snap_hi && (long long)img_m * p.isnap < p.it1) img_it = img_m * p.isnap;
+        } else {
+            img_m = min(p.snap_hi, (p.nt - 1 - it) / p.isnap);
+            if (img_m >= p.snap_lo) img_it = p.nt - 1 - img_m * p.isnap;
+        }
+    }
     if (DIR == 1 && p.img_chip) {
         move_images(true);
-        const int m = min((p.nt - 1 - it) / p.isnap, p.snap_hi);  // the first imaging time is m * isnap
-        if (m >= p.snap_lo && m * p.isnap >= p.nt - p.it1) fetch_snapshot(m - p.snap_base);
+        if (img_it < p.it1) fetch_snapshot(img_m - p.snap_base);
     }
     while (it < p.it1) {
         // steps of this block: up to H, ending at a checked step
@@ -851,10 +854,8 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             // exchange blk: send the frame, collect the halo
             const unsigned tag = p.tag0 + (unsigned)blk;
             const int row0 = my_row0(), col = my_col(), nx = info->nx;
-            const unsigned own = rows_own(row0, nx);
-            const bool lo = lane_owned(col);
             uint4 *const box = p.outbox + (size_t)(blk & 1) * L::BOX;  // this exchange's outbox of CTA 0
-            if (lo) {
+            if (own) {
                 const bool side = lane < RES_HALO || lane >= 32 - RES_HALO;
                 const int ol = lane - RES_HALO / 2;
 #pragma unroll
@@ -1016,18 +1017,12 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 if (p.keep_every && (it + 1 - p.it0) % p.keep_every == 0 && it + 1 < p.nt)
                     store_state(((it + 1 - p.it0) / p.keep_every - 1) * p.keep);
             }
-            if (phase == 0) {
-                const int m = t / p.isnap;
-                if (m >= p.snap_lo && m <= p.snap_hi) {
-                    snapshot(m - p.snap_base);
-                    // the next one's copies are under way while the steps up to it run
-                    if (DIR == 1 && p.img_chip && m - 1 >= p.snap_lo && (m - 1) * p.isnap >= p.nt - p.it1)
-                        fetch_snapshot(m - 1 - p.snap_base);
-                }
-            }
-            if (p.isnap > 0) {
-                if constexpr (DIR == 0) phase = phase + 1 == p.isnap ? 0 : phase + 1;
-                else phase = phase == 0 ? p.isnap - 1 : phase - 1;
+            if (it == img_it) {
+                snapshot(img_m - p.snap_base);
+                img_m += DIR == 0 ? 1 : -1;
+                img_it = (DIR == 0 ? img_m <= p.snap_hi : img_m >= p.snap_lo) && p.isnap < p.it1 - it ? it + p.isnap : p.it1;
+                // the next one's copies are under way while the steps up to it run
+                if (DIR == 1 && p.img_chip && img_it < p.it1) fetch_snapshot(img_m - p.snap_base);
             }
             if (it == next_check) check(it + 1);
             __syncthreads();
