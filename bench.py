@@ -232,8 +232,13 @@ def plain_single_shot(args, rank):
         p = mk(tune, nt)
         p.set_model(*cfg.material(migration=True))
         return p
-    tune = dict(autotune.best_shape(make, cfg.nz, geo, modes, cfg.nt) or {}, graphs=1)
+    tune = dict(graphs=1)  # the library's choice where the shot fits on the chip, as BatchedRTM does
     true = mk(tune, cfg.nt)
+    resident = true.resident()
+    if not resident:
+        true.close()
+        tune = dict(autotune.best_shape(make, cfg.nz, geo, modes, cfg.nt) or {}, graphs=1)
+        true = mk(tune, cfg.nt)
     true.set_model(*cfg.material())
     wav = torch.as_tensor(sh.wavelets).cuda()
     _, obs, _, _ = true.forward(wav)
@@ -263,7 +268,7 @@ def plain_single_shot(args, rank):
     cells = cfg.nx * cfg.nz
     # both modes advanced, as the reference always does (the skipped mode is
     # all zeros here, so the images are the same; this is its cost)
-    pb = Plan(cfg.nx, cfg.nz, cfg.dx, cfg.dz, cfg.nt, cfg.fs, cfg.fw, PSV | SH, geo, tune=tune)
+    pb = Plan(cfg.nx, cfg.nz, cfg.dx, cfg.dz, cfg.nt, cfg.fs, cfg.fw, PSV | SH, geo, tune=dict(graphs=1))
     pb.set_model(*cfg.material(migration=True))
     snaps_b = [pb.snapshot_buffer(nsnap) for _ in range(3)]
 
@@ -297,7 +302,8 @@ def plain_single_shot(args, rank):
                 vs_baseline=None, dtype="f32", data="synthetic",
                 config=dict(workload=cfg.name + f": {cfg.nx}x{cfg.nz}, nt={cfg.nt}, isnap={isnap}, one shot, "
                             "forward with snapshots + backward with imaging"),
-                launch_shape=tune, clocks=clocks, gcell_upd_per_s=round(2 * cells * cfg.nt / (ms / 1000.0) / 1e9, 2),
+                launch_shape=tune, resident=bool(resident), clocks=clocks,
+                gcell_upd_per_s=round(2 * cells * cfg.nt / (ms / 1000.0) / 1e9, 2),
                 us_per_step=round(ms * 1000.0 / (2 * cfg.nt), 2),
                 both_modes=dict(shots_per_s=round(1000.0 / ms_both, 3),
                                 note="P-SV and SH both advanced, as the reference does"),
