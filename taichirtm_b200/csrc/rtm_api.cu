@@ -722,7 +722,8 @@ int resident_setup(rtm_plan *p, bool surface) {
     const int ntz = (p->g.nz + ow - 1) / ow;
     rtm_plan::Resident best;
     std::vector<int4> tiles, stiles;
-    double best_us = streaming_us(p->g.modes, p->rows_total, p->g.nz);
+    const double stream_us = streaming_us(p->g.modes, p->rows_total, p->g.nz);
+    double best_us = stream_us;
     for (int li = 0; li < (int)(sizeof RES_LAYOUTS / sizeof *RES_LAYOUTS); ++li) {
         const ResLayout &lay = RES_LAYOUTS[li];
         if (lay.mode != p->g.modes) continue;
@@ -796,7 +797,13 @@ int resident_setup(rtm_plan *p, bool surface) {
         }
         double us = 0;
         for (int left : room) us += lay.us[(capacity - left + sms - 1) / sms - 1];
-        if (us >= best_us) continue;
+        // The table holds bare steps.  Imaging and checkpoint segments cost the resident
+        // loop more than the streaming one, per launch of tiles, so a P-SV batch in
+        // several launches has to look better by that: of 60 batches of 0.2 to 11
+        // million cells, those at a ratio up to 0.72 took 0.39 to 0.92 of the best
+        // streaming shape's time, those above 0.81 to 1.21.  (SH batches stay below
+        // 0.66, both wave types below 0.97 at any ratio.)
+        if (us >= best_us || (p->g.modes == RTM_PSV && bins.size() > 1 && us > 0.72 * stream_us)) continue;
         best_us = us;
         best = rtm_plan::Resident();
         tiles.clear();
