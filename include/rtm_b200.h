@@ -79,7 +79,8 @@ typedef struct {
     int warps;      /* warps per CTA */
     int prefetch;   /* 1: software-pipelined row loads; 3: cp.async pipeline, rows 3 ahead in a
                        per-warp shared-memory ring (with tsteps 2: the material and 1/rho rows
-                       through a 4-row ring, forward the state rows through a 3-row one); 2: row loads plus L2 cache
+                       through a 4-row ring, in large forward launches that keep their warps with
+                       it the state rows through a 3-row one); 2: row loads plus L2 cache
                        policies (state evict-first, material evict-last); 4: as 3 with tsteps 2, one
                        warp per CTA and the task taken from the block index (warps is set to 1);
                        0: plain; other values = default (1) */

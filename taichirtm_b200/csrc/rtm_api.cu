@@ -4,6 +4,8 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
+#include <atomic>
+#include <climits>
 #include <cstdarg>
 #include <cstdint>
 #include <cmath>
@@ -314,13 +316,14 @@ int run_loop(rtm_plan *p, rtm_plan::GraphCache &gc, const std::vector<unsigned l
 
 unsigned long long U(const void *ptr) { return (unsigned long long)(uintptr_t)ptr; }
 
+constexpr size_t kMaxSmem = 227 * 1024;  // dynamic shared memory of a CTA, opt-in limit
+
 template <int DIR, int MODE, int VEC, int PFM>
 cudaError_t launch_step(const StepParams &sp, int warps, cudaStream_t s) {
     const int threads = 32 * warps;
     const int blocks = (sp.n_work + warps - 1) / warps;
     size_t smem = 0;
     if constexpr (PFM == 3) {
-        constexpr size_t kMaxSmem = 227 * 1024;  // per-block opt-in limit
         smem = (size_t)warps * async_smem_per_warp<MODE, VEC>();
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
         static bool attr_set = false;  // per instantiation; raises the 48 KB default
@@ -366,24 +369,72 @@ cudaError_t launch_mode(const StepParams &sp, int modes, int vec, int warps, cud
     }
 }
 
-template <int DIR, int MODE, int VEC, bool RING, bool STOREA = false, bool CKPT = false, bool UNI = false>
-cudaError_t launch_step2(const StepParams &sp, int warps, cudaStream_t s) {
+// May this kernel have as much shared memory as a CTA can?  Once per instantiation.
+template <int DIR, int MODE, int VEC, bool STOREA, bool CKPT, bool UNI, bool SR>
+cudaError_t ring2_allow_smem() {
+    static std::atomic<bool> done{false};
+    if (done) return cudaSuccess;
+    const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<SR, MODE, VEC>(true), kMaxSmem);
+    const cudaError_t e = cudaFuncSetAttribute(step2_kernel<DIR, MODE, VEC, true, STOREA, CKPT, UNI, SR>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+    done = e == cudaSuccess;
+    return e;
+}
+
+// Warps of this kernel that an SM holds, 0 where a CTA's rings do not fit.
+template <int MODE, int VEC, bool STOREA, bool CKPT, bool UNI, bool SR>
+int ring2_warps_per_sm(int warps, bool surface) {
+    const size_t smem = (size_t)warps * ring2_smem_per_warp<SR, MODE, VEC>(surface);
+    int ctas = 0;
+    if (smem > kMaxSmem || ring2_allow_smem<0, MODE, VEC, STOREA, CKPT, UNI, SR>() != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, step2_kernel<0, MODE, VEC, true, STOREA, CKPT, UNI, SR>, 32 * warps, smem) != cudaSuccess)
+        return 0;
+    return ctas * warps;
+}
+
+// Does a forward ring launch bring the state through a ring too?  Its time against
+// rolling registers, 12 shots of 801 x 801 (2,184 to 8,568 tasks): vec 4, P-SV 0.93
+// to 1.04 and both wave types 0.95 to 1.0 where the SM keeps at least 7/8 of its
+// warps; 1.10 to 1.18 (P-SV, 4 warps, mask: 8 of 12) and 1.47 (both, 4 of 8) where
+// it does not.  With vec 2 a row is short for its copies: P-SV 0.89 to 1.0, with a
+// mask 1.08 to 1.20, both wave types 1.20 to 1.25.  Launches of up to 800 tasks, a
+// wave or two, are bound by the chain of rows: 1.0 to 1.15.
+template <int MODE, int VEC, bool STOREA, bool CKPT, bool UNI>
+bool ring2_state_ring(const StepParams &sp, int warps) {
+    const bool surface = sp.surface != nullptr;
+    if (VEC == 2 && MODE == RTM_PSV && surface) return false;
+    static std::atomic<int> least[9][2];  // per CTA size and mask: tasks from which it is taken, 0: not asked yet
+    int n = least[warps][surface].load();
+    if (n == 0) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+        const int with = ring2_warps_per_sm<MODE, VEC, STOREA, CKPT, UNI, true>(warps, surface);
+        const int without = ring2_warps_per_sm<MODE, VEC, STOREA, CKPT, UNI, false>(warps, surface);
+        n = 8 * with >= 7 * without && with > 0 ? 12 * sms : INT_MAX;
+        least[warps][surface] = n;
+    }
+    return sp.n_work >= n;
+}
+
+template <int DIR, int MODE, int VEC, bool RING, bool STOREA, bool CKPT, bool UNI, bool SR>
+cudaError_t launch_step2_as(const StepParams &sp, int warps, cudaStream_t s) {
     size_t smem = 0;
     if constexpr (RING) {
-        constexpr size_t kMaxSmem = 227 * 1024;  // per-block opt-in limit
-        smem = (size_t)warps * ring2_smem_per_warp<DIR, MODE, VEC>(sp.surface != nullptr);
+        smem = (size_t)warps * ring2_smem_per_warp<SR, MODE, VEC>(sp.surface != nullptr);
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
-        static bool attr_set = false;  // per instantiation; raises the 48 KB default
-        if (!attr_set) {
-            const size_t want = std::min<size_t>(8 * ring2_smem_per_warp<DIR, MODE, VEC>(true), kMaxSmem);
-            cudaError_t e = cudaFuncSetAttribute(step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
-            if (e != cudaSuccess) return e;
-            attr_set = true;
-        }
+        if (const cudaError_t e = ring2_allow_smem<DIR, MODE, VEC, STOREA, CKPT, UNI, SR>()) return e;
     }
-    step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI><<<(sp.n_work + warps - 1) / warps, 32 * warps, smem, s>>>(sp);
+    step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, SR><<<(sp.n_work + warps - 1) / warps, 32 * warps, smem, s>>>(sp);
     return cudaGetLastError();
+}
+
+template <int DIR, int MODE, int VEC, bool RING, bool STOREA = false, bool CKPT = false, bool UNI = false>
+cudaError_t launch_step2(const StepParams &sp, int warps, cudaStream_t s) {
+    if constexpr (RING && DIR == 0 && !(VEC == 2 && MODE == RTM_BOTH)) {
+        if (ring2_state_ring<MODE, VEC, STOREA, CKPT, UNI>(sp, warps))
+            return launch_step2_as<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, true>(sp, warps, s);
+    }
+    return launch_step2_as<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, false>(sp, warps, s);
 }
 
 // Checkpoint-storing forward P-SV launches (sp.ck set): one step or two
@@ -394,7 +445,6 @@ cudaError_t launch_step_ckpt(const StepParams &sp, int warps, cudaStream_t s) {
     const int blocks = (sp.n_work + warps - 1) / warps;
     size_t smem = 0;
     if constexpr (PFM == 3) {
-        constexpr size_t kMaxSmem = 227 * 1024;
         smem = (size_t)warps * async_smem_per_warp<RTM_PSV, VEC>();
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
         static bool attr_set = false;

@@ -123,16 +123,17 @@ __device__ __forceinline__ void ldv_coherent(float (&v)[VEC], float *p) {
 constexpr int RING2_ROWS = 4;
 template <int MODE>
 __host__ __device__ constexpr int ring2_fields() { return ((MODE & 1) ? 5 : 0) + ((MODE & 2) ? 3 : 0); }
-// Forward launches bring the state rows through a ring of their own, three rows
-// deep, too: two rows ahead instead of one, and 20 registers (vec 4) fewer
-// copies per row.  64 shots of 801 columns, vec 4: 166.4 -> 183.7 Gcell/s.
-// Backward launches gain nothing from it (154.6 -> 156.7, and 14 shots lose: 128
-// -> 125) and keep the state in registers.
-template <int DIR>
-__host__ __device__ constexpr int ring2_state_rows() { return DIR == 0 ? 3 : 0; }
-template <int DIR, int MODE, int VEC>
+// State ring (SR, forward with RING): the state rows come through a ring of their
+// own, three rows deep: two rows ahead instead of one, and 20 registers (vec 4)
+// fewer copies per row.  launch_step2 takes it where the rings leave nearly as
+// many warps on an SM (64 shots of 801 columns, vec 4: 166.4 -> 183.7 Gcell/s);
+// elsewhere the state rolls through registers.  Backward launches gain nothing
+// from it (154.6 -> 156.7, and 14 shots lose: 128 -> 125).
+template <bool SR>
+__host__ __device__ constexpr int ring2_state_rows() { return SR ? 3 : 0; }
+template <bool SR, int MODE, int VEC>
 __host__ __device__ constexpr size_t ring2_smem_per_warp(bool surface) {
-    return ((size_t)RING2_ROWS * (ring2_fields<MODE>() + (surface ? 1 : 0)) + ring2_state_rows<DIR>() * ring2_fields<MODE>()) * 32 * VEC * sizeof(float);
+    return ((size_t)RING2_ROWS * (ring2_fields<MODE>() + (surface ? 1 : 0)) + ring2_state_rows<SR>() * ring2_fields<MODE>()) * 32 * VEC * sizeof(float);
 }
 
 // STOREA: also store step A's state (rows [ia, ib), into p.souta), for the
@@ -144,10 +145,11 @@ __host__ __device__ constexpr size_t ring2_smem_per_warp(bool surface) {
 // choices) is then provably the same for the whole warp, so the compiler
 // keeps it in uniform registers and branches on it without divergence
 // bookkeeping; the arithmetic of every cell is unchanged.
-template <int DIR, int MODE, int VEC, bool RING = false, bool STOREA = false, bool CKPT = false, bool UNI = false>
+template <int DIR, int MODE, int VEC, bool RING = false, bool STOREA = false, bool CKPT = false, bool UNI = false, bool SR = false>
 __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams p) {
     static_assert(VEC >= 2, "two steps per launch need two halo columns per side");
     static_assert(!STOREA || DIR == 0, "only the forward recompute stores step A");
+    static_assert(!SR || (DIR == 0 && RING), "the state ring is the forward kernel's");
     static_assert(!CKPT || (DIR == 0 && MODE == 1), "checkpoint stores are forward P-SV");
     constexpr bool PSV = (MODE & 1) != 0;
     constexpr bool SH = (MODE & 2) != 0;
@@ -235,7 +237,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     static_assert((RING2_ROWS & (RING2_ROWS - 1)) == 0, "the ring slot is the row modulo a power of two");
     // this lane's VEC floats of slot 0, field 0; a (slot, field) is a fixed
     // 32-bit offset from it (rows >= -2: row & (RING2_ROWS - 1) is the slot)
-    float *const ring = step2_smem + (UNI ? 0 : (int)(threadIdx.x >> 5) * ((RING2_ROWS * nrf + ring2_state_rows<DIR>() * NRF) * 32 * VEC)) + lane * VEC;
+    float *const ring = step2_smem + (UNI ? 0 : (int)(threadIdx.x >> 5) * ((RING2_ROWS * nrf + ring2_state_rows<SR>() * NRF) * 32 * VEC)) + lane * VEC;
     float *const sring = ring + RING2_ROWS * nrf * (32 * VEC);
     auto rslot = [&](int row, int f) { return ring + ((row & (RING2_ROWS - 1)) * nrf + f) * (32 * VEC); };
     // state ring: slot 0, 1, 2 of the rows in turn; fields as NFIELD of the modes
@@ -654,17 +656,30 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             // iteration k: A velocity k, A stress k-1, B velocity k-1, B stress k-2;
             // ring rows read: k (1/rho), k-1 (1/rho, material), k-2 (material);
             // issued: row k+1 into the slot of row k-3
-            // copy groups in order: material k, state k+1, material k+1, state k+2
+            // SR: copy groups in order: material k, state k+1, material k+1, state k+2
+            if constexpr (!SR) { load_sig(ia - 1, n_so); load_vel(ia - 1, n_vo); }
             ring_issue(ia - 2);
-            state_issue(0, ia - 1);
+            if constexpr (SR) state_issue(0, ia - 1);
             ring_issue(ia - 1);
-            state_issue(1, ia);
+            if constexpr (SR) state_issue(1, ia);
             for (int k = ia - 1; k <= ib + 1; ++k) {
+                if constexpr (!SR) {
+                    cp_sig(so_c, n_so);
+                    cp_vel(vo, n_vo);
+                    if (k <= ib) {
+                        load_sig(k + 1, n_so);
+                        load_vel(k + 1, n_vo);
+                    }
+                }
                 ring_issue(k + 1);
-                state_issue(s2, k + 2);
-                cp_async_wait<3>();  // material and state up to row k have landed
-                rd_state(s0, so_c, vo);
-                { const int t = s0; s0 = s1; s1 = s2; s2 = t; }
+                if constexpr (SR) {
+                    state_issue(s2, k + 2);
+                    cp_async_wait<3>();  // material and state up to row k have landed
+                    rd_state(s0, so_c, vo);
+                    { const int t = s0; s0 = s1; s1 = s2; s2 = t; }
+                } else {
+                    cp_async_wait<1>();  // every material row up to k has landed
+                }
                 {
                     Vel ir;
                     ring_ir(k, ir);

@@ -1,0 +1,79 @@
+"""Launch shapes and the states of a plan that callers can reach: every accepted
+shape runs, with the results of the one-step kernel (tolerance 0), whichever
+form of a kernel and whichever path the library takes for it."""
+import numpy as np
+import pytest
+import torch
+
+from tests.test_gpu_resident import _model, _points, _run, _same, _wavelets
+
+pytestmark = pytest.mark.gpu
+STREAM = dict(vec=2, rows=5, warps=2, tsteps=1)
+
+
+def _topography(nx, nz):
+    surface = np.ones((nx, nz), np.float32)
+    surface[: nx // 2, :2] = 0
+    return surface
+
+
+@pytest.mark.parametrize("modes", [1, 2, 3])
+@pytest.mark.parametrize("vec", [2, 4])
+@pytest.mark.parametrize("warps", [7, 8])
+def test_widest_ring_shapes_run_with_a_mask(modes, vec, warps):
+    """The rings of 8 warps with 4 columns per lane, both wave types and a mask
+    exceed a CTA's shared memory: the state stays in registers then."""
+    from taichirtm_b200.plan import ShotGeometry
+    nx, nz, nt = 70, 130, 8  # no single steps: their kernel has no room for 8 such warps either
+    src, rec = _points(nx, nz, dense=True)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav, mask = _wavelets(len(src), nt), _topography(nx, nz)
+    tune = dict(vec=vec, rows=6, warps=warps, prefetch=3, tsteps=2)
+    a = _run(shots, nx, nz, nt, 12, modes, tune, wav, 2, 0, mask, resident=False)
+    _same(a, _run(shots, nx, nz, nt, 12, modes, STREAM, wav, 2, 0, mask, resident=False))
+
+
+@pytest.mark.parametrize("vec,prefetch,warps", [(2, 3, 2), (2, 4, 1), (4, 3, 4), (4, 4, 1)])
+@pytest.mark.parametrize("modes,mask", [(1, False), (1, True), (2, False), (3, False), (3, True)])
+def test_ring_shapes_with_many_tasks(modes, mask, vec, prefetch, warps):
+    """Launches of 12 tasks per SM and more may bring the state through a ring;
+    the tests on small grids run the other form."""
+    from taichirtm_b200.plan import ShotGeometry
+    nx, nz, nt = 810, 370, 7
+    src, rec = _points(nx, nz, dense=True)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav, surface = _wavelets(len(src), nt), _topography(nx, nz) if mask else None
+    tune = dict(vec=vec, rows=1, warps=warps, prefetch=prefetch, tsteps=2)
+    a = _run(shots, nx, nz, nt, 12, modes, tune, wav, 2, 4, surface, resident=False)
+    _same(a, _run(shots, nx, nz, nt, 12, modes, STREAM, wav, 2, 4, surface, resident=False))
+
+
+@pytest.mark.parametrize("vec", [2, 4])
+@pytest.mark.parametrize("store", ["f32", "i16"])
+def test_ring_checkpoints_and_recompute_with_many_tasks(store, vec):
+    """The storing forms of the same launches: checkpoints, the states that the
+    adjoint recomputes, and what is made of them."""
+    import ctypes
+    from taichirtm_b200 import _lib
+    from taichirtm_b200.plan import Plan, ShotGeometry, _i32p, _ptr, _stream, check as ok
+    nx, nz, nt, every = 810, 370, 11, 5
+    src, rec = _points(nx, nz, dense=False)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav = torch.as_tensor(_wavelets(len(src), nt)).cuda()
+    L, dt, res = _lib.lib(), _lib.CKPT_DTYPES[store], []
+    for tune in (dict(vec=vec, rows=1, warps=2, tsteps=2, prefetch=3), dict(STREAM, vec=vec)):
+        p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 12, 1, shots, tune=tune)
+        p.set_model(*_model(nx, nz))
+        ck = torch.zeros(int(L.rtm_plan_checkpoint_bytes(p.h, every, dt)), dtype=torch.uint8, device="cuda")
+        seis = torch.zeros((3, p.nrec_total, nt), device="cuda")
+        stack = torch.zeros((3, nx, nz), dtype=torch.float64, device="cuda")
+        grad = torch.zeros((5, nx, nz), dtype=torch.float64, device="cuda")
+        flags = np.zeros(1, np.int32)
+        ok(L.rtm_forward_checkpointed(p.h, _ptr(wav), _ptr(seis), every, dt, _ptr(ck), 4, _i32p(flags), _stream()), "f")
+        ok(L.rtm_backward_checkpointed(p.h, _ptr(wav), _ptr(seis), every, dt, _ptr(ck), 2, None, _ptr(stack), 4, _i32p(flags),
+                                       _stream()), "b")
+        ok(L.rtm_adjoint(p.h, _ptr(wav), _ptr(seis), every, dt, _ptr(ck), _ptr(grad), ctypes.c_void_p(0), _stream()), "a")
+        res.append([x.cpu().numpy() for x in (seis, ck, stack, grad)])
+        p.close()
+    assert np.abs(res[0][2]).max() > 0 and np.abs(res[0][3]).max() > 0
+    _same(*res)
