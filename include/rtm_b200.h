@@ -107,6 +107,17 @@ int rtm_plan_destroy(rtm_plan *plan);
  * window fits; results do not depend on it. */
 int rtm_plan_resident(const rtm_plan *plan);
 
+/* Waits of a resident plan.  Its tiles wait for one another; a wait that runs out
+ * (after some seconds) ends the launch with incomplete results.  Entry points that
+ * synchronise (flags not NULL, rtm_backward_normalized, rtm_adjoint,
+ * rtm_backward_checkpointed) then return RTM_E_CUDA.  rtm_forward, rtm_backward and
+ * rtm_forward_checkpointed with flags NULL return before the GPU is done: theirs is
+ * reported by the next call on the plan that synchronises, or by rtm_plan_status,
+ * which waits for `stream`, writes the shots' status codes of the last call to flags
+ * (host, may be NULL) and returns RTM_E_CUDA for such a wait since the last report.
+ * No reference counterpart. */
+int rtm_plan_status(rtm_plan *plan, int32_t *flags, rtm_stream_t stream);
+
 /* Floats per padded row of the internal layout (row i at (i+1)*pitch + 4). */
 int rtm_plan_pitch(const rtm_plan *plan);
 /* Floats of ONE snapshot component for all shots of the plan and nsnap
@@ -310,6 +321,10 @@ const char *rtm_version(void);
  * aid standing in for a memory checker). */
 int rtm_bounds_probe(const rtm_plan *plan, const void *buf, size_t buf_bytes, const void *ptr, size_t bytes,
                      int32_t *inside);
+/* Also of that build: a wait between the tiles of a resident plan runs out after
+ * this many polls in later calls (<= 0: the default), so that a test sees it
+ * reported.  The normal build returns RTM_E_STATE. */
+int rtm_plan_set_wait_limit(rtm_plan *plan, int polls);
 
 #ifdef __cplusplus
 }

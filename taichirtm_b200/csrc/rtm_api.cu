@@ -172,6 +172,7 @@ struct rtm_plan {
         void *base = nullptr;     // their allocation
     } res;
     bool auto_shape = false;  // the launch shape is the library's choice
+    int wait_limit = RES_SPIN_LIMIT;  // rtm_plan_set_wait_limit (bounds-checking build)
     std::vector<int> src_ptr_h, rec_ptr_h;  // host copies of the row tables
     std::vector<int2> src_ent_h, rec_ent_h;
 };
@@ -254,7 +255,7 @@ struct BoundsScope {
         add(p->d_rec_ptr, p->n_rec_ptr * sizeof(int));
         add(p->d_src_ent, p->n_src_ent * sizeof(int2));
         add(p->d_rec_ent, p->n_rec_ent * sizeof(int2));
-        add(p->d_flags, (p->nshots + 1) * sizeof(int));
+        add(p->d_flags, (p->nshots + 2) * sizeof(int));
         add(p->d_fail_seq, p->nshots * sizeof(int));
         add(p->res.d_box, p->res.box_bytes);
         add(p->d_sponge, (size_t)std::max(p->g.absorbing_frame, 1) * F);
@@ -582,7 +583,7 @@ void fill_common(const rtm_plan *p, StepParams &sp) {
 }
 
 int zero_status(rtm_plan *p, cudaStream_t s) {
-    CUDA_TRY(cudaMemsetAsync(p->d_flags, 0, (p->nshots + 1) * sizeof(int), s));
+    CUDA_TRY(cudaMemsetAsync(p->d_flags, 0, (p->nshots + 1) * sizeof(int), s));  // not the second error word: read_status
     CUDA_TRY(cudaMemsetAsync(p->d_fail_seq, 0x7f, p->nshots * sizeof(int), s));  // 0x7f7f7f7f: none
     return 0;
 }
@@ -594,15 +595,18 @@ int zero_state(rtm_plan *p, cudaStream_t s) {
     return zero_status(p, s);
 }
 
-// The per-shot status codes to host memory (synchronises), and the resident
-// kernel's error word behind them.
+// The per-shot status codes to host memory (synchronises), and the second of the
+// resident kernel's error words behind them.  That one stays set until it has been
+// reported: calls with null flags return before the GPU is done and cannot.
 int read_status(rtm_plan *p, int32_t *flags, cudaStream_t s) {
-    std::vector<int> h(p->nshots + 1);
+    const int n = p->nshots;
+    std::vector<int> h(n + 2);
     CUDA_TRY(cudaMemcpyAsync(h.data(), p->d_flags, h.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
-    std::copy(h.begin(), h.begin() + p->nshots, flags);
-    if (h[p->nshots]) return fail(RTM_E_CUDA, "resident propagation: a wait between tiles ran out");
-    return 0;
+    if (flags) std::copy(h.begin(), h.begin() + n, flags);
+    if (!h[n + 1]) return 0;
+    CUDA_TRY(cudaMemsetAsync(p->d_flags + n + 1, 0, sizeof(int), s));
+    return fail(RTM_E_CUDA, "resident propagation: a wait between tiles ran out, in this call or in one since the last reported status");
 }
 
 // ---- resident propagation (resident_kernels.cuh)
@@ -710,6 +714,9 @@ void resident_params(const rtm_plan *p, ResParams &rp, int dir) {
     rp.flags = p->d_flags;
     rp.fail_seq = p->d_fail_seq;
     rp.err = p->d_flags + p->nshots;
+#ifdef RTM_BOUNDS_CHECK
+    rp.polls0 = RES_SPIN_LIMIT - p->wait_limit;
+#endif
     for (int f = 0; f < NFIELD; ++f) rp.store[f] = p->d_state[0][f];
     rp.tiles = p->res.d_tiles;
     rp.shot_tiles = p->res.d_shot_tiles;
@@ -1088,7 +1095,7 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     p->n_rec_ptr = rec_ptr.size();
     p->n_src_ent = std::max<size_t>(src_ent.size(), 1);
     p->n_rec_ent = std::max<size_t>(rec_ent.size(), 1);
-    p->slab.add(&p->d_flags, (size_t)nshots + 1);  // the last word: the resident kernel's error
+    p->slab.add(&p->d_flags, (size_t)nshots + 2);  // the last words: ResParams::err
     p->slab.add(&p->d_fail_seq, nshots);
     p->slab.add(&p->d_sponge, std::max(g.absorbing_frame, 1));
     for (int b = 0; b < 2; ++b)
@@ -1124,6 +1131,7 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     if (e == cudaSuccess) e = H2D(p->d_src_ent, src_ent.data(), src_ent.size() * sizeof(int2));
     if (e == cudaSuccess) e = H2D(p->d_rec_ent, rec_ent.data(), rec_ent.size() * sizeof(int2));
     if (e == cudaSuccess) e = H2D(p->d_sponge, prof.data(), prof.size() * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemset(p->d_flags, 0, ((size_t)nshots + 2) * sizeof(int));
     if (e != cudaSuccess) {
         plan_free(p);
         delete p;
@@ -1145,6 +1153,22 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
 }
 
 int rtm_plan_resident(const rtm_plan *p) { return p && p->res.layout >= 0 ? 1 : 0; }
+
+int rtm_plan_set_wait_limit(rtm_plan *p, int polls) {
+    if (!p) return fail(RTM_E_ARG, "null plan");
+#ifdef RTM_BOUNDS_CHECK
+    p->wait_limit = polls > 0 ? std::min(polls, RES_SPIN_LIMIT) : RES_SPIN_LIMIT;
+    return RTM_OK;
+#else
+    (void)polls;
+    return fail(RTM_E_STATE, "rtm_plan_set_wait_limit needs the bounds-checking build (-DRTM_BOUNDS_CHECK)");
+#endif
+}
+
+int rtm_plan_status(rtm_plan *p, int32_t *flags, rtm_stream_t stream) {
+    if (!p) return fail(RTM_E_ARG, "null plan");
+    return read_status(p, flags, (cudaStream_t)stream);
+}
 
 int rtm_plan_destroy(rtm_plan *p) {
     if (!p) return RTM_OK;
@@ -1542,11 +1566,8 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
             ++p->launches;
         }
     }
-    if (flags) {
+    if (flags || norm)  // norm: the slot table is host memory of this call
         if (int rc = read_status(p, flags, s)) return rc;
-    } else if (norm) {
-        CUDA_TRY(cudaStreamSynchronize(s));  // the slot table is host memory of this call
-    }
     if (int rc = bs.end(s)) return rc;
     return RTM_OK;
 }
@@ -2014,8 +2035,7 @@ int rtm_adjoint(rtm_plan *p, const float *wavelets, const float *resid, int ckpt
         if (gwt) {
             if (int r = transpose(gwt, grad_wavelet, 3, nt, p->nsrc_total, s)) return r;
         }
-        std::vector<int> status(p->nshots);
-        if (int r = read_status(p, status.data(), s)) return r;
+        if (int r = read_status(p, nullptr, s)) return r;
         if (int r = bs.end(s)) return r;
         return RTM_OK;
     };
@@ -2223,8 +2243,7 @@ int rtm_backward_checkpointed(rtm_plan *p, const float *wavelets, const float *o
                     CUDA_TRY(cudaGetLastError());
                 }
         }
-        std::vector<int32_t> status(p->nshots);  // the call waits for its results in any case
-        if (int rc = read_status(p, flags ? flags : status.data(), s)) return rc;
+        if (int rc = read_status(p, flags, s)) return rc;  // the call waits for its results in any case
         if (int rc = bs.end(s)) return rc;
         return RTM_OK;
     };

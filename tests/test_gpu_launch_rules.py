@@ -77,3 +77,54 @@ def test_ring_checkpoints_and_recompute_with_many_tasks(store, vec):
         p.close()
     assert np.abs(res[0][2]).max() > 0 and np.abs(res[0][3]).max() > 0
     _same(*res)
+
+
+WAIT = r'''
+import numpy as np, torch
+from taichirtm_b200 import _lib
+from taichirtm_b200._lib import RtmError, check as ok
+from taichirtm_b200.plan import Plan, ShotGeometry, _i32p, _ptr, _stream
+from tests.test_gpu_resident import _model, _points, _wavelets
+nx, nz, nt = 300, 150, 40
+src, rec = _points(nx, nz, dense=False)
+p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 20, 1, [ShotGeometry(0, nx, src, rec)])
+p.set_model(*_model(nx, nz))
+assert p.resident()
+L, wav = _lib.lib(), torch.as_tensor(_wavelets(len(src), nt)).cuda()
+want = p.forward(wav)[1].clone()
+seis, flags, none = torch.zeros_like(want), np.zeros(1, np.int32), None
+
+def forward(flags):
+    return L.rtm_forward(p.h, _ptr(wav), _ptr(seis), 0, 1, none, none, none, none, 0, flags, _stream())
+
+def status():
+    return L.rtm_plan_status(p.h, _i32p(flags), _stream())
+
+assert forward(none) == 0 and status() == 0 and torch.equal(seis, want)
+ok(L.rtm_plan_set_wait_limit(p.h, 1), "limit")
+forward(none)
+assert status() == -2 and b"ran out" in L.rtm_last_error()
+assert status() == 0  # reported once
+assert forward(_i32p(flags)) == -2 and status() == 0
+try:
+    p.backward(want, None, [], 0, 1)
+    raise SystemExit("backward reported nothing")
+except RtmError:
+    pass
+forward(none)
+ok(L.rtm_plan_set_wait_limit(p.h, 0), "limit")
+forward(none)  # complete itself, and does not hide the one before
+assert status() == -2 and torch.equal(seis, want)
+assert forward(_i32p(flags)) == 0 and torch.equal(seis, want)
+print("WAIT_OK")
+'''
+
+
+def test_wait_that_runs_out_is_reported():
+    """A wait limit of one poll (bounds-checking build): no packet of a neighbouring
+    tile is there by then, so the tiles leave at their first exchange and the
+    results are incomplete.  Calls with flags say so; the others leave it to the
+    next report."""
+    from tests.test_gpu_bounds import _child
+    r = _child(WAIT, timeout=300)
+    assert r.returncode == 0 and "WAIT_OK" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
