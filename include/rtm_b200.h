@@ -72,7 +72,8 @@ typedef struct {
 /* Kernel launch shape (autotuned by the Python layer).  With NULL, or vec, rows,
  * warps and tsteps 0 and prefetch <= 0, the library chooses: a wavefield that
  * fits on the chip stays there (rtm_plan_resident), others stream with a shape
- * that follows from the grid.  Results do not depend on any of it. */
+ * that follows from the grid (for prefetch 0 and nothing else, set tsteps 1).
+ * Results do not depend on any of it. */
 typedef struct {
     int vec;        /* columns per lane: 1, 2 or 4 */
     int rows;       /* rows per warp task (the tasks a launch dispatches last get half as many) */

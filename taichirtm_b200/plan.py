@@ -64,6 +64,10 @@ class Plan:
             self._keep += [s.src, s.rec]
             arr[k] = _lib.RtmShot(s.x0, s.nx, len(s.src), _i32p(s.src), len(s.rec), _i32p(s.rec))
         t = tune or {}
+        if t.get("prefetch", -1) == 0 and not any(t.get(k) for k in ("vec", "rows", "warps", "tsteps")):
+            # prefetch 0 by itself asks for plain row loads; all zeros would leave
+            # the whole shape to the library (a zero-initialised rtm_tune)
+            t = dict(t, tsteps=1)
         tn = _lib.RtmTune(int(t.get("vec", 0)), int(t.get("rows", 0)), int(t.get("warps", 0)),
                           int(t.get("prefetch", -1)), int(t.get("graphs", 0)), int(t.get("tsteps", 0)))
         h = ctypes.c_void_p()

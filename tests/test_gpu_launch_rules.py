@@ -79,6 +79,18 @@ def test_ring_checkpoints_and_recompute_with_many_tasks(store, vec):
     _same(*res)
 
 
+def test_prefetch_zero_is_a_launch_shape():
+    """prefetch 0 by itself asks for plain row loads, so the plan streams; a negative
+    one, like no launch shape at all, leaves the choice to the library."""
+    from taichirtm_b200.plan import ShotGeometry
+    nx, nz, nt = 40, 30, 6
+    src, rec = _points(nx, nz, dense=False)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav = _wavelets(len(src), nt)
+    a = _run(shots, nx, nz, nt, 4, 3, dict(prefetch=0), wav, 2, 0, resident=False)
+    _same(a, _run(shots, nx, nz, nt, 4, 3, dict(prefetch=-1, graphs=1), wav, 2, 0, resident=True))
+
+
 WAIT = r'''
 import numpy as np, torch
 from taichirtm_b200 import _lib
