@@ -298,7 +298,8 @@ const char *rtm_noalloc_last_error(void);
 typedef int (*rtm_step_callback)(void *user, int step);
 int rtm_plan_set_callback(rtm_plan *plan, int forward_every, rtm_step_callback cb, void *user);
 /* The velocity wavefield of one shot as the last step of rtm_forward /
- * rtm_backward left it (during a step callback: after that step), copied to
+ * rtm_backward left it (during a step callback: after that step; of a shot that
+ * stopped: after the step whose check failed), copied to
  * dense (nx_shot, nz) DEVICE arrays u, v, w (any may be NULL; a component the
  * plan does not propagate is written as zeros).  RTM_E_STATE before any
  * rtm_forward / rtm_backward, or after a checkpointed entry point. */

@@ -6,6 +6,8 @@
 
 namespace rtm {
 
+constexpr int NEVER_FAILED = 0x7f7f7f7f;  // fail_seq of a shot that runs to the end
+
 // ForwardModeling._compute_shear_avg / _compute_rho_avg / _compute_inv_rho
 // (forward_modeling.py:243-307) into the padded layout, evaluated in double
 // and rounded once to float.  The reference's f32 form multiplies four
@@ -143,6 +145,18 @@ static __global__ void illum_kernel(const float *__restrict__ snap, const int *_
     }
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(imax + blockIdx.y, (unsigned long long)__double_as_longlong(m));
+}
+
+// One field of one shot's window (at `off` in a state buffer) to a dense (nx, nz)
+// array: from `live`, the buffer number `parity`, or, where the shot stopped at
+// launch *fail_seq, from the buffer of that launch's parity.
+static __global__ void wavefield_kernel(const float *live, const float *other, int parity, const int *fail_seq,
+                                        long long off, int nx, int nz, int pitch, float *dst) {
+    const int f = fail_seq ? *fail_seq : NEVER_FAILED;
+    const float *src = (f != NEVER_FAILED && (f & 1) != parity ? other : live) + off;
+    const long long n = (long long)nx * nz;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+        dst[k] = src[(k / nz) * pitch + k % nz];
 }
 
 }  // namespace rtm

@@ -155,6 +155,9 @@ struct rtm_plan {
     void *cb_user = nullptr;
     int cb_every = 0;
     int live = -1;
+    // fail_seq counts launches: a stopped shot's latest state is in the buffer
+    // that the launch of that number wrote, not in `live`
+    bool live_seq = false;
     // Resident propagation (resident_kernels.cuh): the tile layout chosen at
     // plan creation, or r == 0 when the plan streams its wavefield.
     struct Resident {
@@ -1211,9 +1214,10 @@ int rtm_plan_wavefield(const rtm_plan *p, int shot, float *u, float *v, float *w
             CUDA_TRY(cudaMemsetAsync(dst[c], 0, (size_t)d.nx * nz * sizeof(float), s));
             continue;
         }
-        CUDA_TRY(cudaMemcpy2DAsync(dst[c], (size_t)nz * sizeof(float), src + d.state_off + p->pitch + COL_OFF,
-                                   (size_t)p->pitch * sizeof(float), (size_t)nz * sizeof(float), (size_t)d.nx,
-                                   cudaMemcpyDeviceToDevice, s));
+        wavefield_kernel<<<(int)std::min<long long>(((long long)d.nx * nz + 255) / 256, 148LL * 16), 256, 0, s>>>(
+            src, p->d_state[1 - p->live][field[c]], p->live, p->live_seq ? p->d_fail_seq + shot : nullptr,
+            d.state_off + p->pitch + COL_OFF, d.nx, nz, p->pitch, dst[c]);
+        CUDA_TRY(cudaGetLastError());
     }
     return RTM_OK;
 }
@@ -1324,7 +1328,7 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
                 sp.sout[f] = p->d_state[(L + 1) & 1][f];
             }
             sp.it = it;
-            sp.seq = it + 1;
+            sp.seq = (int)L + 1;  // its last bit: the buffer that the launch writes
             sp.snap_k = snap_at(it);
             const int last = sched[L].two ? it + 1 : it;
             if (sched[L].two) {
@@ -1337,8 +1341,9 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
                 CUDA_TRY((launch_mode<0>(sp, p->g.modes, p->vec | (std::min(p->prefetch, 3) << 8), p->warps, ls)));
             }
             p->live = (int)((L + 1) & 1);
+            p->live_seq = true;
             if (cb_at(last))
-                if (int rc = call_back(p, it + 1, last, ls)) return rc;
+                if (int rc = call_back(p, sp.seq, last, ls)) return rc;
         }
         return 0;
     };
@@ -1365,12 +1370,16 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
         if (int rc = resident_begin(p, s)) return rc;
         if (int rc = resident_run(p, rp, 0, s)) return rc;
         p->live = 0;
+        p->live_seq = false;
     } else if (p->cb) {  // host callbacks in the loop: direct launches
         if (int rc = loop(s)) return rc;
     } else if (int rc = run_loop(p, p->g_fwd, key, s, loop)) {
         return rc;
     }
-    if (!resident) p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
+    if (!resident) {  // also when a replayed graph ran the loop
+        p->live = (int)(sched.size() & 1);
+        p->live_seq = true;
+    }
     p->launches += (long long)sched.size();
     if (seis && p->nrec_total) {
         if (int rc = transpose(p->d_seis_t, seis, 3, nt, p->nrec_total, s)) return rc;
@@ -1463,7 +1472,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
                 sp.sout[f] = p->d_state[(L + 1) & 1][f];
             }
             sp.it = (nt - 1) - it;  // backward_modeling.py:549
-            sp.seq = it + 1;
+            sp.seq = (int)L + 1;
             sp.snap_k = snap_of[it];
             const int last = sched[L].two ? it + 1 : it;
             if (sched[L].two) {
@@ -1476,8 +1485,9 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
                 CUDA_TRY((launch_mode<1>(sp, p->g.modes, p->vec | (std::min(p->prefetch, 3) << 8), p->warps, ls)));
             }
             p->live = (int)((L + 1) & 1);
+            p->live_seq = true;
             if (cb_at(last))
-                if (int rc = call_back(p, it + 1, (nt - 1) - last, ls)) return rc;
+                if (int rc = call_back(p, sp.seq, (nt - 1) - last, ls)) return rc;
         }
         return 0;
     };
@@ -1506,12 +1516,16 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
         if (int rc = resident_begin(p, s)) return rc;
         if (int rc = resident_run(p, rp, 1, s)) return rc;
         p->live = 0;
+        p->live_seq = false;
     } else if (p->cb) {  // host callbacks in the loop: direct launches
         if (int rc = loop(s)) return rc;
     } else if (int rc = run_loop(p, p->g_bwd, key, s, loop)) {
         return rc;
     }
-    if (!resident) p->live = (int)(sched.size() & 1);  // also when a replayed graph ran the loop
+    if (!resident) {  // also when a replayed graph ran the loop
+        p->live = (int)(sched.size() & 1);
+        p->live_seq = true;
+    }
     p->launches += (long long)sched.size();
     const int blocks = 148 * 8;
     const size_t n = (size_t)p->g.nx * p->g.nz;

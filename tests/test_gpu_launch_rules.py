@@ -91,6 +91,36 @@ def test_prefetch_zero_is_a_launch_shape():
     _same(a, _run(shots, nx, nz, nt, 4, 3, dict(prefetch=-1, graphs=1), wav, 2, 0, resident=True))
 
 
+@pytest.mark.parametrize("tune", [None, dict(vec=2, rows=5, warps=2, tsteps=1), dict(vec=2, rows=5, warps=2, tsteps=2),
+                                  dict(vec=4, rows=5, warps=1, tsteps=2, prefetch=4, graphs=1)])
+@pytest.mark.parametrize("nt,check", [(12, 1), (13, 3), (14, 5), (14, 3)])
+def test_wavefield_of_a_stopped_shot(tune, nt, check):
+    """The wavefield of a shot that stopped is the one of its last step, the step
+    whose check failed, however the plan runs; other shots go on to the end."""
+    from taichirtm_b200.plan import Plan, ShotGeometry
+    nx, nz, w, fw, at = 90, 40, 50, 5, 3
+    rec = np.array([[i, 1] for i in range(w)], np.int32)
+    shots = [ShotGeometry(0, w, np.array([[25, 20]], np.int32), rec), ShotGeometry(40, w, np.array([[25, 20]], np.int32), rec)]
+    # dt dx dz / rho of it, 1e33, is above the check's limit of 1e30 at step `at`
+    wav = _wavelets(2, nt)
+    wav[:, 0, at] = 3e38
+    last = -(-at // check) * check
+    mu, lam, rho = _model(nx, nz)
+    p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, fw, 1, shots, tune=tune)
+    p.set_model(mu, lam, rho)
+    flags, _, _, _ = p.forward(torch.as_tensor(wav), check_interval=check)
+    assert flags[0] > 0 and flags[1] == 0
+    got = [p.wavefield(k).cpu().numpy() for k in range(2)]
+    p.close()
+    # the same shots by themselves, over the steps each ran, without checks
+    for k, steps in ((0, last + 1), (1, nt)):
+        q = Plan(nx, nz, 4.0, 4.0, steps, 2000.0, fw, 1, [shots[k]], tune=STREAM)
+        q.set_model(mu, lam, rho)
+        q.forward(torch.as_tensor(np.ascontiguousarray(wav[:, k:k + 1, :steps])), check_interval=0)
+        assert np.array_equal(got[k], q.wavefield(0).cpu().numpy(), equal_nan=True)
+        q.close()
+
+
 WAIT = r'''
 import numpy as np, torch
 from taichirtm_b200 import _lib
