@@ -1349,7 +1349,7 @@ int rtm_forward(rtm_plan *p, const float *wavelets, float *seis, int save, int i
     };
     const std::vector<unsigned long long> key = {U(wavelets), U(snap_u), U(snap_v), U(snap_w),
                                                  (unsigned long long)save, (unsigned long long)isnap,
-                                                 (unsigned long long)check_interval};
+                                                 (unsigned long long)check_interval, U(sp.surface)};
     if (resident) {
         ResParams rp;
         resident_params(p, rp, 0);
@@ -1492,7 +1492,7 @@ static int backward_impl(rtm_plan *p, const float *obs, const float *snap_u, con
         return 0;
     };
     std::vector<unsigned long long> key = {U(snap_u), U(snap_v), U(snap_w), (unsigned long long)num_snaps,
-                                           (unsigned long long)isnap, (unsigned long long)check_interval};
+                                           (unsigned long long)isnap, (unsigned long long)check_interval, U(sp.surface)};
     for (int it = 0; it < nt; ++it)
         if (snap_of[it] >= 0) key.push_back(((unsigned long long)it << 32) | (unsigned)snap_of[it]);
     if (resident) {

@@ -121,6 +121,68 @@ def test_wavefield_of_a_stopped_shot(tune, nt, check):
         q.close()
 
 
+@pytest.mark.parametrize("modes", [1, 3])
+@pytest.mark.parametrize("tune", [dict(vec=2, rows=9, warps=2, tsteps=2, graphs=1), dict(vec=2, rows=9, warps=2, tsteps=2, prefetch=3, graphs=1),
+                                  dict(vec=4, rows=9, warps=2, tsteps=1, graphs=1), None])
+def test_mask_added_and_dropped_on_one_plan(tune, modes):
+    """set_model decides whether there is a mask, also after loops that were
+    captured or laid out for the other case."""
+    from taichirtm_b200.plan import Plan, ShotGeometry
+    nx, nz, nt = 90, 75, 11
+    src, rec = _points(nx, nz, dense=True)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav = torch.as_tensor(_wavelets(len(src), nt)).cuda()
+    model, mask = _model(nx, nz), _topography(nx, nz)
+
+    def passes(p, snaps=None):
+        out = []
+        f, seis, snaps, isn = p.forward(wav, save=True, isnap=2, check_interval=0, snaps=snaps)
+        _, img, _ = p.backward(seis, snaps, isn, len(isn), 2, check_interval=0)
+        return [seis.cpu().numpy(), img.cpu().numpy()], snaps
+
+    want = {}
+    for has in (False, True):
+        q = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 8, modes, shots, tune=STREAM)
+        q.set_model(*model, mask if has else None)
+        want[has], _ = passes(q)
+        q.close()
+    assert not np.array_equal(want[False][0], want[True][0])
+    p, snaps = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 8, modes, shots, tune=tune), None
+    for has in (False, True, False, True, True, False):
+        p.set_model(*model, mask if has else None)
+        got, snaps = passes(p, snaps)
+        _same(got, want[has])
+    assert p.resident() == (tune is None)
+    p.close()
+
+
+
+@pytest.mark.parametrize("tune", [dict(vec=2, rows=9, warps=2, tsteps=2), dict(vec=4, rows=9, warps=2, tsteps=1, prefetch=3)])
+def test_graph_replays_of_streaming_plans(tune):
+    """Time loops captured once and replayed give what direct launches give: on the
+    capturing call, on replays with other data in the same buffers, and after the
+    snapshot schedule has changed and changed back."""
+    from taichirtm_b200.plan import Plan, ShotGeometry
+    nx, nz, nt = 90, 75, 17
+    src, rec = _points(nx, nz, dense=True)
+    res = []
+    for graphs in (0, 1):
+        p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 8, 3, [ShotGeometry(0, nx, src, rec)], tune=dict(tune, graphs=graphs))
+        p.set_model(*_model(nx, nz))
+        assert not p.resident()
+        wav = torch.empty((3, len(src), nt), device="cuda")
+        bufs, out = {i: [p.snapshot_buffer(nt // i) for _ in range(3)] for i in (2, 3)}, []
+        for seed, isnap in ((1, 2), (2, 2), (3, 3), (4, 3), (5, 2)):
+            wav.copy_(torch.as_tensor(_wavelets(len(src), nt, seed)))
+            f, seis, snaps, isn = p.forward(wav, save=True, isnap=isnap, check_interval=4, snaps=bufs[isnap])
+            fb, img, _ = p.backward(seis, snaps, isn, len(isn), isnap, check_interval=4)
+            out += [f, fb, seis.cpu().numpy(), img.cpu().numpy()] + [p.snapshot_view(b, len(isn)).cpu().numpy() for b in snaps]
+        res.append(out)
+        p.close()
+    assert np.abs(res[0][2]).max() > 0 and np.abs(res[0][3]).max() > 0
+    _same(*res)
+
+
 WAIT = r'''
 import numpy as np, torch
 from taichirtm_b200 import _lib
