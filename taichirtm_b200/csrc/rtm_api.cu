@@ -174,6 +174,10 @@ struct rtm_plan {
         std::vector<int2> waves;  // (first tile, tiles) of each launch
         void *base = nullptr;     // their allocation
     } res;
+    // The layouts made so far, without and with a mask, kept until the plan is
+    // destroyed: a call that a caller captured goes on using its layout's buffers.
+    Resident laid[2];
+    bool is_laid[2] = {false, false};
     bool auto_shape = false;  // the launch shape is the library's choice
     int wait_limit = RES_SPIN_LIMIT;  // rtm_plan_set_wait_limit (bounds-checking build)
     std::vector<int> src_ptr_h, rec_ptr_h;  // host copies of the row tables
@@ -203,7 +207,8 @@ int plan_scratch(rtm_plan *p, size_t n, float **out) {
 
 void plan_free(rtm_plan *p) {
     p->slab.release();
-    if (p->res.base) cudaFree(p->res.base);
+    for (auto &r : p->laid)
+        if (r.base) cudaFree(r.base);
     if (p->d_scratch) cudaFree(p->d_scratch);
     for (auto *gc : {&p->g_fwd, &p->g_bwd, &p->g_ckpt})
         if (gc->exec) cudaGraphExecDestroy(gc->exec);
@@ -768,9 +773,12 @@ int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
 // estimated step is shortest, and build its tables.  Leaves p->res.layout at -1
 // when there is none, or when streaming is estimated to be faster.
 int resident_setup(rtm_plan *p, bool surface) {
+    if (p->is_laid[surface]) {
+        p->res = p->laid[surface];
+        return 0;
+    }
     const std::vector<int> &src_ptr = p->src_ptr_h, &rec_ptr = p->rec_ptr_h;
     const std::vector<int2> &src_ent = p->src_ent_h, &rec_ent = p->rec_ent_h;
-    if (p->res.base) cudaFree(p->res.base);
     p->res = rtm_plan::Resident();
     p->res.surface = surface;
     int dev = 0, sms = 0, coop = 0;
@@ -883,8 +891,12 @@ int resident_setup(rtm_plan *p, bool surface) {
         best.max_rec_all = max_rec_all;
         best.max_rec = max_rec;
     }
-    if (best.layout < 0) return 0;
     best.surface = surface;
+    if (best.layout < 0) {
+        p->laid[surface] = best;
+        p->is_laid[surface] = true;
+        return 0;
+    }
     p->res = best;
     int box = 0;
     resident_smem(RES_LAYOUTS[best.layout], 0, 0, false, &box);
@@ -901,9 +913,16 @@ int resident_setup(rtm_plan *p, bool surface) {
         p->res = rtm_plan::Resident();
         return rc;
     }
+    cudaError_t e = cudaMemcpy(p->res.d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(p->res.d_shot_tiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        slab.release();
+        p->res = rtm_plan::Resident();
+        return fail(RTM_E_CUDA, "upload of the tiles failed: %s", cudaGetErrorString(e));
+    }
     p->res.base = slab.base;
-    CUDA_TRY(cudaMemcpy(p->res.d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(p->res.d_shot_tiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    p->laid[surface] = p->res;
+    p->is_laid[surface] = true;
     return 0;
 }
 
@@ -1239,8 +1258,16 @@ int rtm_plan_set_model(rtm_plan *p, const float *mu, const float *lam, const flo
         p->d_mat[M_MYZ], surface ? p->d_surface : nullptr);
     CUDA_TRY(cudaGetLastError());
     p->has_surface = surface != nullptr;
-    if (p->auto_shape && p->has_surface != p->res.surface)
-        if (int rc = resident_setup(p, p->has_surface)) return rc;
+    if (p->auto_shape && (p->has_surface != p->res.surface || !p->is_laid[p->has_surface])) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+        if (capture != cudaStreamCaptureStatusNone && !p->is_laid[p->has_surface]) {
+            p->res = rtm_plan::Resident();  // nothing can be allocated now: stream until the next set_model
+            p->res.surface = p->has_surface;
+        } else if (int rc = resident_setup(p, p->has_surface)) {
+            return rc;
+        }
+    }
     p->model_set = true;
     return RTM_OK;
 }

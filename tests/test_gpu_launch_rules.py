@@ -183,6 +183,55 @@ def test_graph_replays_of_streaming_plans(tune):
     _same(*res)
 
 
+
+def test_captured_calls_outlive_a_change_of_the_mask():
+    """A forward call that a caller captured (flags NULL) replays after set_model has
+    added a mask, with the buffers and the maskless loop it was captured with.  A
+    set_model that meets a mask for the first time can be captured, too."""
+    from taichirtm_b200 import _lib
+    from taichirtm_b200._lib import check as ok
+    from taichirtm_b200.plan import Plan, ShotGeometry, _ptr, _stream
+    nx, nz, nt = 300, 150, 21
+    src, rec = _points(nx, nz, dense=False)
+    shots, L = [ShotGeometry(0, nx, src, rec)], _lib.lib()
+    model = [torch.as_tensor(x).cuda() for x in _model(nx, nz)]
+    mask, wav = torch.as_tensor(_topography(nx, nz)).cuda(), torch.as_tensor(_wavelets(len(src), nt)).cuda()
+    want = {}
+    for has in (False, True):
+        q = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 20, 3, shots, tune=STREAM)
+        q.set_model(*model, mask if has else None)
+        want[has] = q.forward(wav)[1]
+        q.close()
+    assert not torch.equal(want[False], want[True])
+    p, seis, none = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 20, 3, shots), torch.zeros_like(want[False]), None
+
+    def call():
+        ok(L.rtm_forward(p.h, _ptr(wav), _ptr(seis), 0, 1, none, none, none, none, 0, none, _stream()), "rtm_forward")
+
+    def replay(graph):
+        seis.zero_()
+        graph.replay()
+        ok(L.rtm_plan_status(p.h, none, _stream()), "rtm_plan_status")
+        return seis
+    p.set_model(*model)
+    assert p.resident() and torch.equal(p.forward(wav)[1], want[False])
+    plain, masked = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(plain):
+        call()
+    assert torch.equal(replay(plain), want[False])
+    with torch.cuda.graph(masked):
+        p.set_model(*model, mask)
+        call()
+    assert not p.resident() and torch.equal(replay(masked), want[True])
+    p.set_model(*model, mask)
+    assert p.resident() and torch.equal(p.forward(wav)[1], want[True])
+    assert torch.equal(replay(plain), want[False]) and torch.equal(replay(masked), want[True])
+    p.set_model(*model)
+    assert p.resident() and torch.equal(p.forward(wav)[1], want[False])
+    del plain, masked
+    p.close()
+
+
 WAIT = r'''
 import numpy as np, torch
 from taichirtm_b200 import _lib
