@@ -104,8 +104,9 @@ int rtm_plan_destroy(rtm_plan *plan);
 /* 1 when the plan keeps its wavefield on the chip: one launch (or a few, when
  * its shots do not all fit at once) then runs a whole time loop.  The plan
  * chooses it at creation when rtm_tune leaves the launch shape to the library
- * (NULL, or vec, rows, warps and tsteps 0 and prefetch <= 0) and every shot's
- * window fits; results do not depend on it. */
+ * (NULL, or vec, rows, warps and tsteps 0 and prefetch <= 0), every shot's window
+ * fits and the device memory left holds its buffers; rtm_plan_set_model chooses
+ * again when a mask comes or goes.  Results do not depend on it. */
 int rtm_plan_resident(const rtm_plan *plan);
 
 /* Waits of a resident plan.  Its tiles wait for one another; a wait that runs out

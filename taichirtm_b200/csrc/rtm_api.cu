@@ -771,7 +771,8 @@ int resident_run(rtm_plan *p, ResParams &rp, int dir, cudaStream_t s) {
 
 // Choose the layout in which every shot's tiles are resident together and the
 // estimated step is shortest, and build its tables.  Leaves p->res.layout at -1
-// when there is none, or when streaming is estimated to be faster.
+// when there is none, when streaming is estimated to be faster, or when the
+// device memory left does not hold its buffers.
 int resident_setup(rtm_plan *p, bool surface) {
     if (p->is_laid[surface]) {
         p->res = p->laid[surface];
@@ -909,9 +910,11 @@ int resident_setup(rtm_plan *p, bool surface) {
     slab.add(&p->res.d_shot_tiles, stiles.size());
     slab.add(&p->res.d_sync, 2 * (size_t)p->nshots);
     slab.add(&p->res.d_box, p->res.box_bytes / sizeof(uint4));
-    if (int rc = slab.commit()) {
+    if (slab.commit()) {
+        cudaGetLastError();  // no room: the plan streams, the next set_model tries again
         p->res = rtm_plan::Resident();
-        return rc;
+        p->res.surface = surface;
+        return 0;
     }
     cudaError_t e = cudaMemcpy(p->res.d_tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(p->res.d_shot_tiles, stiles.data(), stiles.size() * sizeof(int4), cudaMemcpyHostToDevice);

@@ -232,6 +232,41 @@ def test_captured_calls_outlive_a_change_of_the_mask():
     p.close()
 
 
+def test_plan_streams_when_its_resident_buffers_do_not_fit():
+    """A plan whose own buffers fit in the device memory that is left, but not
+    those of the resident loops too, is made all the same and streams."""
+    from taichirtm_b200.plan import Plan, ShotGeometry
+    nx, nz, nt = 560, 700, 6
+    src, rec = _points(nx, nz, dense=False)
+    shots = [ShotGeometry(0, nx, src, rec)]
+    wav, model = torch.as_tensor(_wavelets(len(src), nt)).cuda(), [torch.as_tensor(x).cuda() for x in _model(nx, nz)]
+
+    def make(tune):
+        p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 20, 1, shots, tune=tune)
+        p.set_model(*model)
+        return p
+
+    def used(tune):  # device memory that a plan of this shape takes
+        before = torch.cuda.mem_get_info()[0]
+        p = make(tune)
+        n, resident = before - torch.cuda.mem_get_info()[0], p.resident()
+        seis = p.forward(wav)[1]
+        p.close()
+        return n, resident, seis
+
+    used(None)  # one-time loading of the kernels
+    (n_stream, r_stream, want), (n_res, r_res, seis) = used(STREAM), used(None)
+    assert r_res and not r_stream and torch.equal(want, seis) and n_res - n_stream > 16 << 20
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (n_stream + n_res) // 2, dtype=torch.uint8, device="cuda")
+    p = make(None)
+    resident = p.resident()
+    del hold
+    torch.cuda.empty_cache()
+    assert not resident and torch.equal(p.forward(wav)[1], want)
+    p.close()
+
+
 WAIT = r'''
 import numpy as np, torch
 from taichirtm_b200 import _lib
