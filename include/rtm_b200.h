@@ -84,7 +84,8 @@ typedef struct {
                        it the state rows through a 3-row one); 2: row loads plus L2 cache
                        policies (state evict-first, material evict-last); 4: as 3 with tsteps 2, one
                        warp per CTA and the task taken from the block index (warps is set to 1);
-                       0: plain; other values = default (1) */
+                       0: plain; other values = default (1).  With tsteps 2, both wave types and
+                       vec 4 the rows always take the ring (they would spill) */
     int graphs;     /* 1: capture each time loop as a CUDA graph on first use and replay it
                        while its pointers and schedule stay the same; 0 = direct launches */
     int tsteps;     /* time steps per launch of rtm_forward, rtm_backward and the

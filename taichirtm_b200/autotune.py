@@ -73,7 +73,7 @@ def _store(cache):
 def key(nz, shots, modes):
     name = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     rows = sum(s.nx for s in shots)
-    return f"{name}|nz={nz}|rows={rows}|shots={len(shots)}|modes={modes}|v13"
+    return f"{name}|nz={nz}|rows={rows}|shots={len(shots)}|modes={modes}|v14"
 
 
 def time_shape(make_plan, shots, tune, steps=TUNE_STEPS):

@@ -42,4 +42,21 @@ __device__ __forceinline__ f2 f2_sel(bool lo, bool hi, f2 a, f2 b) {
     return f2_pack(lo ? f2_lo(a) : f2_lo(b), hi ? f2_hi(a) : f2_hi(b));
 }
 
+// Two lanes of arithmetic on an f2: packed instructions, or two scalar ones (for
+// kernels that lose more to the even register pairs than packing saves).
+template <bool PACKED>
+struct Pairs {
+    static __device__ __forceinline__ f2 pack(float lo, float hi) { return f2_pack(lo, hi); }
+    static __device__ __forceinline__ f2 add(f2 a, f2 b) { return f2_add(a, b); }
+    static __device__ __forceinline__ f2 sub(f2 a, f2 b) { return f2_sub(a, b); }
+    static __device__ __forceinline__ f2 mul(f2 a, f2 b, f2 neg_zero) { return f2_mul(a, b, neg_zero); }
+};
+template <>
+struct Pairs<false> {
+    static __device__ __forceinline__ f2 pack(float lo, float hi) { return (f2)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
+    static __device__ __forceinline__ f2 add(f2 a, f2 b) { return pack(f2_lo(a) + f2_lo(b), f2_hi(a) + f2_hi(b)); }
+    static __device__ __forceinline__ f2 sub(f2 a, f2 b) { return pack(f2_lo(a) - f2_lo(b), f2_hi(a) - f2_hi(b)); }
+    static __device__ __forceinline__ f2 mul(f2 a, f2 b, f2) { return pack(f2_lo(a) * f2_lo(b), f2_hi(a) * f2_hi(b)); }
+};
+
 }  // namespace rtm

@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <climits>
 #include <cstdarg>
 #include <cstdint>
 #include <cmath>
@@ -390,6 +389,18 @@ cudaError_t ring2_allow_smem() {
     return e;
 }
 
+// Enough tasks to be bound by what a task costs rather than by its chain of rows?
+bool many_tasks(const StepParams &sp) {
+    static std::atomic<int> least{0};
+    int n = least.load();
+    if (n == 0) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+        least = n = 12 * sms;
+    }
+    return sp.n_work >= n;
+}
+
 // Warps of this kernel that an SM holds, 0 where a CTA's rings do not fit.
 template <int MODE, int VEC, bool STOREA, bool CKPT, bool UNI, bool SR>
 int ring2_warps_per_sm(int warps, bool surface) {
@@ -412,17 +423,16 @@ template <int MODE, int VEC, bool STOREA, bool CKPT, bool UNI>
 bool ring2_state_ring(const StepParams &sp, int warps) {
     const bool surface = sp.surface != nullptr;
     if (VEC == 2 && MODE == RTM_PSV && surface) return false;
-    static std::atomic<int> least[9][2];  // per CTA size and mask: tasks from which it is taken, 0: not asked yet
-    int n = least[warps][surface].load();
-    if (n == 0) {
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    if (!many_tasks(sp)) return false;
+    static std::atomic<int> keeps[9][2];  // per CTA size and mask: 1 yes, -1 no, 0 not asked yet
+    int k = keeps[warps][surface].load();
+    if (k == 0) {
         const int with = ring2_warps_per_sm<MODE, VEC, STOREA, CKPT, UNI, true>(warps, surface);
         const int without = ring2_warps_per_sm<MODE, VEC, STOREA, CKPT, UNI, false>(warps, surface);
-        n = 8 * with >= 7 * without && with > 0 ? 12 * sms : INT_MAX;
-        least[warps][surface] = n;
+        k = 8 * with >= 7 * without && with > 0 ? 1 : -1;
+        keeps[warps][surface] = k;
     }
-    return sp.n_work >= n;
+    return k > 0;
 }
 
 template <int DIR, int MODE, int VEC, bool RING, bool STOREA, bool CKPT, bool UNI, bool SR>
@@ -433,7 +443,23 @@ cudaError_t launch_step2_as(const StepParams &sp, int warps, cudaStream_t s) {
         if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
         if (const cudaError_t e = ring2_allow_smem<DIR, MODE, VEC, STOREA, CKPT, UNI, SR>()) return e;
     }
-    step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, SR><<<(sp.n_work + warps - 1) / warps, 32 * warps, smem, s>>>(sp);
+    const int blocks = (sp.n_work + warps - 1) / warps;
+    // Many tasks hide the longer chain of packed operations: P-SV, 8,568 tasks 1.01,
+    // 800 tasks 0.98 of packed with scalar ones (a gradient of 8 shots of 1201 x 401
+    // 79.3 against 78.5 ms)
+    if constexpr (MODE == RTM_PSV && VEC == 2 && !RING) {
+        if (many_tasks(sp)) {
+            step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, SR, 8, true><<<blocks, 32 * warps, smem, s>>>(sp);
+            return cudaGetLastError();
+        }
+    }
+    if constexpr (MODE == RTM_SH && VEC == 2 && !RING) {  // 12 shots of 801 x 801, 4 warps: 51.5 -> 44.8 us per step
+        if (warps <= 4) {
+            step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, SR, 4><<<blocks, 32 * warps, smem, s>>>(sp);
+            return cudaGetLastError();
+        }
+    }
+    step2_kernel<DIR, MODE, VEC, RING, STOREA, CKPT, UNI, SR><<<blocks, 32 * warps, smem, s>>>(sp);
     return cudaGetLastError();
 }
 
@@ -503,7 +529,10 @@ cudaError_t launch_vec2(const StepParams &sp, int vec, bool ring, bool uni, int 
                         : launch_step2<DIR, MODE, 4, true, false, false, true>(sp, 1, s);
     }
     if (vec == 2) return ring ? launch_step2<DIR, MODE, 2, true>(sp, warps, s) : launch_step2<DIR, MODE, 2, false>(sp, warps, s);
-    return ring ? launch_step2<DIR, MODE, 4, true>(sp, warps, s) : launch_step2<DIR, MODE, 4, false>(sp, warps, s);
+    // both wave types, vec 4: rolling registers spill (12 shots of 801 x 801, 4 warps:
+    // 117 us per step, 85 through the ring), so the ring kernel runs them all
+    if constexpr (MODE == RTM_BOTH) return launch_step2<DIR, MODE, 4, true>(sp, warps, s);
+    else return ring ? launch_step2<DIR, MODE, 4, true>(sp, warps, s) : launch_step2<DIR, MODE, 4, false>(sp, warps, s);
 }
 
 // Forward recompute of the adjoint, P-SV: steps sp.it and sp.it2 in one

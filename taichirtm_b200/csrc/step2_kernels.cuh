@@ -83,13 +83,13 @@ __device__ __forceinline__ void unpack(float (&d)[2 * N], const f2 (&s)[N]) {
     for (int q = 0; q < N; ++q) { d[2 * q] = f2_lo(s[q]); d[2 * q + 1] = f2_hi(s[q]); }
 }
 // Differences with the next lower / higher column; nb: the neighbouring lane's.
-template <int N>
+template <class A, int N>
 __device__ __forceinline__ f2 diff_lo(const f2 (&x)[N], int q, float nb) {
-    return f2_pack(f2_lo(x[q]) - (q > 0 ? f2_hi(x[q > 0 ? q - 1 : 0]) : nb), f2_hi(x[q]) - f2_lo(x[q]));
+    return A::pack(f2_lo(x[q]) - (q > 0 ? f2_hi(x[q > 0 ? q - 1 : 0]) : nb), f2_hi(x[q]) - f2_lo(x[q]));
 }
-template <int N>
+template <class A, int N>
 __device__ __forceinline__ f2 diff_hi(const f2 (&x)[N], int q, float nb) {
-    return f2_pack(f2_hi(x[q]) - f2_lo(x[q]), (q < N - 1 ? f2_lo(x[q < N - 1 ? q + 1 : 0]) : nb) - f2_hi(x[q]));
+    return A::pack(f2_hi(x[q]) - f2_lo(x[q]), (q < N - 1 ? f2_lo(x[q < N - 1 ? q + 1 : 0]) : nb) - f2_hi(x[q]));
 }
 
 // Plain (coherent) vector load for the Kahan image: one thread may read a
@@ -136,17 +136,39 @@ __host__ __device__ constexpr size_t ring2_smem_per_warp(bool surface) {
     return ((size_t)RING2_ROWS * (ring2_fields<MODE>() + (surface ? 1 : 0)) + ring2_state_rows<SR>() * ring2_fields<MODE>()) * 32 * VEC * sizeof(float);
 }
 
+// Packed arithmetic, or scalar?  Scalar against packed, 0.2 to 7.7 million cells:
+// without the rings 0.94 to 1.0 with vec 2 (its two columns are one chain of packed
+// operations where they were two; launch_step2_as has the exception), 1.0 to 1.04 for
+// P-SV and SH with vec 4.  With the material
+// ring and the state in registers 0.92 to 1.0 for P-SV with vec 2 and for SH, 1.0
+// to 1.1 for the rest; with the state ring 1.0 to 1.1.  Backward with the ring 0.96
+// to 1.0 for SH with vec 2, else 0.95 to 1.15 either way.
+__host__ __device__ constexpr bool step2_packed(int dir, int mode, int vec, bool ring, bool state_ring) {
+    if (!ring) return vec == 4 && mode != 3;
+    if (dir == 1) return mode != 2 || vec == 4;
+    return state_ring || mode == 3 || (mode == 1 && vec == 4);
+}
+// CTAs per SM that the register budget is cut for (0: as it comes).  Both wave types
+// backward, vec 2, 8 warps: 140 registers left one CTA on an SM.  SH, vec 2, 4 warps,
+// no ring: 100 to 120 registers left four CTAs where 96, without spills, leave five.
+__host__ __device__ constexpr int step2_min_ctas(int dir, int mode, int vec, bool ring, bool uni, int warps) {
+    if (mode == 3 && vec == 2 && ring && !uni && dir == 1) return 2;
+    return mode == 2 && vec == 2 && !ring && warps == 4 ? 5 : 0;
+}
+
 // STOREA: also store step A's state (rows [ia, ib), into p.souta), for the
 // forward recompute of the FWI adjoint, which needs the state after every step.
 // CKPT: step B's state is also stored, block-scaled to 16 bits, into the
 // checkpoint slot p.ck (ckpt_pack.cuh); forward P-SV only.
+// WARPS: the most warps a CTA is launched with.
 // UNI: launched with one warp per CTA, the task is blockIdx.x.  Everything
 // derived from the task (shot, strip, row range, loop bounds, fast-path
 // choices) is then provably the same for the whole warp, so the compiler
 // keeps it in uniform registers and branches on it without divergence
 // bookkeeping; the arithmetic of every cell is unchanged.
-template <int DIR, int MODE, int VEC, bool RING = false, bool STOREA = false, bool CKPT = false, bool UNI = false, bool SR = false>
-__global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams p) {
+template <int DIR, int MODE, int VEC, bool RING = false, bool STOREA = false, bool CKPT = false, bool UNI = false, bool SR = false, int WARPS = 8,
+          bool PACKED = step2_packed(DIR, MODE, VEC, RING, SR)>
+__global__ void __launch_bounds__(UNI ? 32 : 32 * WARPS, step2_min_ctas(DIR, MODE, VEC, RING, UNI, WARPS)) step2_kernel(const StepParams p) {
     static_assert(VEC >= 2, "two steps per launch need two halo columns per side");
     static_assert(!STOREA || DIR == 0, "only the forward recompute stores step A");
     static_assert(!SR || (DIR == 0 && RING), "the state ring is the forward kernel's");
@@ -154,6 +176,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     constexpr bool PSV = (MODE & 1) != 0;
     constexpr bool SH = (MODE & 2) != 0;
     constexpr int W = 30 * VEC;
+    using A = Pairs<PACKED>;
     using Sig = SigRow<VEC>;
     using Vel = VelRow<VEC>;
     using Mat = MatRow<VEC>;
@@ -195,7 +218,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
     const long long soff = sh.state_off + (long long)(c0 + COL_OFF);
     const long long moff = (long long)sh.x0 * P + (long long)(c0 + COL_OFF);
     const float dt = p.dt, idx = p.inv_dx, idz = p.inv_dz;
-    const f2 dt2 = f2_pack(dt, dt), idx2 = f2_pack(idx, idx), idz2 = f2_pack(idz, idz), nz2 = f2_pack(p.neg_zero, p.neg_zero);
+    const f2 dt2 = A::pack(dt, dt), idx2 = A::pack(idx, idx), idz2 = A::pack(idz, idz), nz2 = A::pack(p.neg_zero, p.neg_zero);
     constexpr int NP = VEC / 2;
     // CKPT: scale block of row -1 of this task's strip (padded row 0 of the shot)
     long long ck_blk0 = 0;
@@ -224,7 +247,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             ldp<NP>(m.sm, p.surface + moff + (long long)(rowc(i) + 1) * P);
         } else {
 #pragma unroll
-            for (int q = 0; q < NP; ++q) m.sm[q] = f2_pack(1.f, 1.f);
+            for (int q = 0; q < NP; ++q) m.sm[q] = A::pack(1.f, 1.f);
         }
     };
     // ---- material ring (RING): slot of a row, copy-in, read-back
@@ -304,7 +327,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             rd_ring(row, RF_SM, m.sm);
         } else {
 #pragma unroll
-            for (int q = 0; q < NP; ++q) m.sm[q] = f2_pack(1.f, 1.f);
+            for (int q = 0; q < NP; ++q) m.sm[q] = A::pack(1.f, 1.f);
         }
     };
     (void)ring_issue; (void)ring_ir; (void)ring_mat;
@@ -348,28 +371,28 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
             if constexpr (PSV) {
-                const f2 sxx_x = f2_mul(f2_sub(sc.xx[q], sp.xx[q]), idx2, nz2);  // fm:332, bm:333
-                const f2 sxz_x = f2_mul(f2_sub(sc.xz[q], sp.xz[q]), idx2, nz2);  // fm:334, bm:335
+                const f2 sxx_x = A::mul(A::sub(sc.xx[q], sp.xx[q]), idx2, nz2);  // fm:332, bm:333
+                const f2 sxz_x = A::mul(A::sub(sc.xz[q], sp.xz[q]), idx2, nz2);  // fm:334, bm:335
                 f2 dzz, dxz;
-                if constexpr (DIR == 0) { dzz = diff_lo(sc.zz, q, zz_nb); dxz = diff_lo(sc.xz, q, xz_nb); }
-                else { dzz = diff_hi(sp.zz, q, zz_nb); dxz = diff_hi(sp.xz, q, xz_nb); }
-                const f2 szz_z = f2_mul(dzz, idz2, nz2);                          // fm:333, bm:334
-                const f2 sxz_z = f2_mul(dxz, idz2, nz2);                          // fm:335, bm:336
-                f2 du = f2_mul(f2_mul(f2_add(sxx_x, sxz_z), dt2, nz2), ir.u[q], nz2);  // fm:339, bm:340 (negated)
-                f2 dw = f2_mul(f2_mul(f2_add(sxz_x, szz_z), dt2, nz2), ir.w[q], nz2);  // fm:340, bm:341
+                if constexpr (DIR == 0) { dzz = diff_lo<A>(sc.zz, q, zz_nb); dxz = diff_lo<A>(sc.xz, q, xz_nb); }
+                else { dzz = diff_hi<A>(sp.zz, q, zz_nb); dxz = diff_hi<A>(sp.xz, q, xz_nb); }
+                const f2 szz_z = A::mul(dzz, idz2, nz2);                          // fm:333, bm:334
+                const f2 sxz_z = A::mul(dxz, idz2, nz2);                          // fm:335, bm:336
+                f2 du = A::mul(A::mul(A::add(sxx_x, sxz_z), dt2, nz2), ir.u[q], nz2);  // fm:339, bm:340 (negated)
+                f2 dw = A::mul(A::mul(A::add(sxz_x, szz_z), dt2, nz2), ir.w[q], nz2);  // fm:340, bm:341
                 if constexpr (!FAST) { du = clip(du, q, rm); dw = clip(dw, q, rm); }
-                out.u[q] = DIR == 0 ? f2_add(vo.u[q], du) : f2_sub(vo.u[q], du);
-                out.w[q] = DIR == 0 ? f2_add(vo.w[q], dw) : f2_sub(vo.w[q], dw);
+                out.u[q] = DIR == 0 ? A::add(vo.u[q], du) : A::sub(vo.u[q], du);
+                out.w[q] = DIR == 0 ? A::add(vo.w[q], dw) : A::sub(vo.w[q], dw);
             }
             if constexpr (SH) {
-                const f2 syx_x = f2_mul(f2_sub(sc.yx[q], sp.yx[q]), idx2, nz2);  // fm:343, bm:343
+                const f2 syx_x = A::mul(A::sub(sc.yx[q], sp.yx[q]), idx2, nz2);  // fm:343, bm:343
                 f2 dyz;
-                if constexpr (DIR == 0) dyz = diff_lo(sc.yz, q, yz_nb);
-                else dyz = diff_hi(sp.yz, q, yz_nb);
-                const f2 syz_z = f2_mul(dyz, idz2, nz2);                          // fm:344, bm:344
-                f2 dv = f2_mul(f2_mul(f2_add(syx_x, syz_z), dt2, nz2), ir.v[q], nz2);  // fm:347, bm:345
+                if constexpr (DIR == 0) dyz = diff_lo<A>(sc.yz, q, yz_nb);
+                else dyz = diff_hi<A>(sp.yz, q, yz_nb);
+                const f2 syz_z = A::mul(dyz, idz2, nz2);                          // fm:344, bm:344
+                f2 dv = A::mul(A::mul(A::add(syx_x, syz_z), dt2, nz2), ir.v[q], nz2);  // fm:347, bm:345
                 if constexpr (!FAST) dv = clip(dv, q, rm);
-                out.v[q] = DIR == 0 ? f2_add(vo.v[q], dv) : f2_sub(vo.v[q], dv);
+                out.v[q] = DIR == 0 ? A::add(vo.v[q], dv) : A::sub(vo.v[q], dv);
             }
         }
     };
@@ -410,7 +433,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                     for (int k = 0; k < NP; ++k) {  // x + -0.0 is x: the other columns take part
                         const float b = q & 1 ? f2_hi(ir2[k]) : f2_lo(ir2[k]);
                         const float a = wf * (in || !masked ? b : __int_as_float(0x7f800000));
-                        x[k] = f2_add(x[k], f2_pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
+                        x[k] = A::add(x[k], A::pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
                     }
                 };
                 if constexpr (PSV) { add(out.u, ir.u, p.wav[0], true); add(out.w, ir.w, p.wav[2], true); }
@@ -428,7 +451,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                     const float a = ldg_chk(obs + ti);
 #pragma unroll
                     for (int k = 0; k < NP; ++k)
-                        x[k] = f2_add(x[k], f2_pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
+                        x[k] = A::add(x[k], A::pack(q == 2 * k ? a : -0.0f, q == 2 * k + 1 ? a : -0.0f));
                 };
                 if constexpr (PSV) { add(out.u, p.obs[0]); add(out.w, p.obs[2]); }
                 if constexpr (SH) add(out.v, p.obs[1]);
@@ -461,7 +484,7 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
             if (ra) cr_i = ldg_chk(p.sponge + r);
             if (rb) cr_dr = ldg_chk(p.sponge + dr);
         }
-        const f2 sdt2 = DIR == 0 ? dt2 : f2_pack(-dt, -dt);
+        const f2 sdt2 = DIR == 0 ? dt2 : A::pack(-dt, -dt);
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
             f2 c = 0ull;
@@ -474,54 +497,54 @@ __global__ void __launch_bounds__(UNI ? 32 : 256) step2_kernel(const StepParams 
                     if (rb && col_db[k] > dr) cr[h] = cr_dr;
                     if (col_sp[k] && r >= col_db[k] && dr >= col_db[k]) cr[h] = col_cr[k];
                 }
-                c = f2_pack(cr[0], cr[1]);
+                c = A::pack(cr[0], cr[1]);
             }
             if constexpr (PSV) {
                 f2 dux, dwx, duz, dwz;
                 if constexpr (DIR == 0) {
-                    dux = f2_sub(vb.u[q], va.u[q]); dwx = f2_sub(vb.w[q], va.w[q]);
-                    duz = diff_hi(va.u, q, nu); dwz = diff_hi(va.w, q, nw);
+                    dux = A::sub(vb.u[q], va.u[q]); dwx = A::sub(vb.w[q], va.w[q]);
+                    duz = diff_hi<A>(va.u, q, nu); dwz = diff_hi<A>(va.w, q, nw);
                 } else {
-                    dux = f2_sub(va.u[q], vb.u[q]); dwx = f2_sub(va.w[q], vb.w[q]);
-                    duz = diff_lo(va.u, q, nu); dwz = diff_lo(va.w, q, nw);
+                    dux = A::sub(va.u[q], vb.u[q]); dwx = A::sub(va.w[q], vb.w[q]);
+                    duz = diff_lo<A>(va.u, q, nu); dwz = diff_lo<A>(va.w, q, nw);
                 }
-                const f2 u_x = f2_mul(dux, idx2, nz2), u_z = f2_mul(duz, idz2, nz2);  // fm:369-370, bm:366-367
-                const f2 w_x = f2_mul(dwx, idx2, nz2), w_z = f2_mul(dwz, idz2, nz2);  // fm:371-372, bm:368-369
-                const f2 ld = f2_mul(m.lam[q], f2_add(u_x, w_z), nz2), mu2 = f2_add(m.mu[q], m.mu[q]);
-                f2 dxx = f2_mul(sdt2, f2_add(ld, f2_mul(mu2, u_x, nz2)), nz2);
-                f2 dzz = f2_mul(sdt2, f2_add(ld, f2_mul(mu2, w_z, nz2)), nz2);
-                f2 dxz = f2_mul(f2_mul(sdt2, m.mxz[q], nz2), f2_add(u_z, w_x), nz2);
+                const f2 u_x = A::mul(dux, idx2, nz2), u_z = A::mul(duz, idz2, nz2);  // fm:369-370, bm:366-367
+                const f2 w_x = A::mul(dwx, idx2, nz2), w_z = A::mul(dwz, idz2, nz2);  // fm:371-372, bm:368-369
+                const f2 ld = A::mul(m.lam[q], A::add(u_x, w_z), nz2), mu2 = A::add(m.mu[q], m.mu[q]);
+                f2 dxx = A::mul(sdt2, A::add(ld, A::mul(mu2, u_x, nz2)), nz2);
+                f2 dzz = A::mul(sdt2, A::add(ld, A::mul(mu2, w_z, nz2)), nz2);
+                f2 dxz = A::mul(A::mul(sdt2, m.mxz[q], nz2), A::add(u_z, w_x), nz2);
                 if constexpr (FAST) {
-                    os.xx[q] = f2_add(base.xx[q], dxx);
-                    os.zz[q] = f2_add(base.zz[q], dzz);
-                    os.xz[q] = f2_add(base.xz[q], dxz);
+                    os.xx[q] = A::add(base.xx[q], dxx);
+                    os.zz[q] = A::add(base.zz[q], dzz);
+                    os.xz[q] = A::add(base.xz[q], dxz);
                     ov.u[q] = va.u[q];
                     ov.w[q] = va.w[q];
                 } else {
                     dxx = clip(dxx, q, rm); dzz = clip(dzz, q, rm); dxz = clip(dxz, q, rm);
-                    os.xx[q] = f2_mul(c, f2_add(base.xx[q], dxx), nz2);
-                    os.zz[q] = f2_mul(f2_mul(c, f2_add(base.zz[q], dzz), nz2), m.sm[q], nz2);
-                    os.xz[q] = f2_mul(f2_mul(c, f2_add(base.xz[q], dxz), nz2), m.sm[q], nz2);
-                    ov.u[q] = f2_mul(c, va.u[q], nz2);
-                    ov.w[q] = f2_mul(c, va.w[q], nz2);
+                    os.xx[q] = A::mul(c, A::add(base.xx[q], dxx), nz2);
+                    os.zz[q] = A::mul(A::mul(c, A::add(base.zz[q], dzz), nz2), m.sm[q], nz2);
+                    os.xz[q] = A::mul(A::mul(c, A::add(base.xz[q], dxz), nz2), m.sm[q], nz2);
+                    ov.u[q] = A::mul(c, va.u[q], nz2);
+                    ov.w[q] = A::mul(c, va.w[q], nz2);
                 }
             }
             if constexpr (SH) {
                 f2 dvx, dvz;
-                if constexpr (DIR == 0) { dvx = f2_sub(vb.v[q], va.v[q]); dvz = diff_hi(va.v, q, nv); }
-                else { dvx = f2_sub(va.v[q], vb.v[q]); dvz = diff_lo(va.v, q, nv); }
-                const f2 v_x = f2_mul(dvx, idx2, nz2), v_z = f2_mul(dvz, idz2, nz2);  // fm:381-382, bm:377-378
-                f2 dyx = f2_mul(f2_mul(sdt2, m.myx[q], nz2), v_x, nz2);
-                f2 dyz = f2_mul(f2_mul(sdt2, m.myz[q], nz2), v_z, nz2);
+                if constexpr (DIR == 0) { dvx = A::sub(vb.v[q], va.v[q]); dvz = diff_hi<A>(va.v, q, nv); }
+                else { dvx = A::sub(va.v[q], vb.v[q]); dvz = diff_lo<A>(va.v, q, nv); }
+                const f2 v_x = A::mul(dvx, idx2, nz2), v_z = A::mul(dvz, idz2, nz2);  // fm:381-382, bm:377-378
+                f2 dyx = A::mul(A::mul(sdt2, m.myx[q], nz2), v_x, nz2);
+                f2 dyz = A::mul(A::mul(sdt2, m.myz[q], nz2), v_z, nz2);
                 if constexpr (FAST) {
-                    os.yx[q] = f2_add(base.yx[q], dyx);
-                    os.yz[q] = f2_add(base.yz[q], dyz);
+                    os.yx[q] = A::add(base.yx[q], dyx);
+                    os.yz[q] = A::add(base.yz[q], dyz);
                     ov.v[q] = va.v[q];
                 } else {
                     dyx = clip(dyx, q, rm); dyz = clip(dyz, q, rm);
-                    os.yx[q] = f2_mul(c, f2_add(base.yx[q], dyx), nz2);
-                    os.yz[q] = f2_mul(f2_mul(c, f2_add(base.yz[q], dyz), nz2), m.sm[q], nz2);
-                    ov.v[q] = f2_mul(c, va.v[q], nz2);
+                    os.yx[q] = A::mul(c, A::add(base.yx[q], dyx), nz2);
+                    os.yz[q] = A::mul(A::mul(c, A::add(base.yz[q], dyz), nz2), m.sm[q], nz2);
+                    ov.v[q] = A::mul(c, va.v[q], nz2);
                 }
             }
         }

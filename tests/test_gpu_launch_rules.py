@@ -33,11 +33,11 @@ def test_widest_ring_shapes_run_with_a_mask(modes, vec, warps):
     _same(a, _run(shots, nx, nz, nt, 12, modes, STREAM, wav, 2, 0, mask, resident=False))
 
 
-@pytest.mark.parametrize("vec,prefetch,warps", [(2, 3, 2), (2, 4, 1), (4, 3, 4), (4, 4, 1)])
+@pytest.mark.parametrize("vec,prefetch,warps", [(2, 3, 2), (2, 4, 1), (4, 3, 4), (4, 4, 1), (2, 1, 4), (2, 1, 8), (4, 1, 4)])
 @pytest.mark.parametrize("modes,mask", [(1, False), (1, True), (2, False), (3, False), (3, True)])
-def test_ring_shapes_with_many_tasks(modes, mask, vec, prefetch, warps):
-    """Launches of 12 tasks per SM and more may bring the state through a ring;
-    the tests on small grids run the other form."""
+def test_shapes_with_many_tasks(modes, mask, vec, prefetch, warps):
+    """Launches of 12 tasks per SM and more may bring the state through a ring, or
+    use packed arithmetic; the tests on small grids run the other forms."""
     from taichirtm_b200.plan import ShotGeometry
     nx, nz, nt = 810, 370, 7
     src, rec = _points(nx, nz, dense=True)
@@ -48,9 +48,9 @@ def test_ring_shapes_with_many_tasks(modes, mask, vec, prefetch, warps):
     _same(a, _run(shots, nx, nz, nt, 12, modes, STREAM, wav, 2, 4, surface, resident=False))
 
 
-@pytest.mark.parametrize("vec", [2, 4])
+@pytest.mark.parametrize("vec,prefetch", [(2, 1), (2, 3), (4, 3)])
 @pytest.mark.parametrize("store", ["f32", "i16"])
-def test_ring_checkpoints_and_recompute_with_many_tasks(store, vec):
+def test_checkpoints_and_recompute_with_many_tasks(store, vec, prefetch):
     """The storing forms of the same launches: checkpoints, the states that the
     adjoint recomputes, and what is made of them."""
     import ctypes
@@ -61,7 +61,7 @@ def test_ring_checkpoints_and_recompute_with_many_tasks(store, vec):
     shots = [ShotGeometry(0, nx, src, rec)]
     wav = torch.as_tensor(_wavelets(len(src), nt)).cuda()
     L, dt, res = _lib.lib(), _lib.CKPT_DTYPES[store], []
-    for tune in (dict(vec=vec, rows=1, warps=2, tsteps=2, prefetch=3), dict(STREAM, vec=vec)):
+    for tune in (dict(vec=vec, rows=1, warps=2, tsteps=2, prefetch=prefetch), dict(STREAM, vec=vec)):
         p = Plan(nx, nz, 4.0, 4.0, nt, 2000.0, 12, 1, shots, tune=tune)
         p.set_model(*_model(nx, nz))
         ck = torch.zeros(int(L.rtm_plan_checkpoint_bytes(p.h, every, dt)), dtype=torch.uint8, device="cuda")
