@@ -110,6 +110,11 @@ int rtm_plan_destroy(rtm_plan *plan);
  * again when a mask comes or goes.  Results do not depend on it. */
 int rtm_plan_resident(const rtm_plan *plan);
 
+/* How a resident plan is laid out (host, 5 values): rows per lane of its P-SV and of
+ * its SH tiles (0: no such tiles), warps per tile, launches per time loop, and
+ * whether rtm_backward keeps the images on the chip.  RTM_E_STATE for other plans. */
+int rtm_plan_resident_layout(const rtm_plan *plan, int32_t *layout);
+
 /* Waits of a resident plan.  Its tiles wait for one another; a wait that runs out
  * (after some seconds) ends the launch with incomplete results.  Entry points that
  * synchronise (flags not NULL, rtm_backward_normalized, rtm_adjoint,

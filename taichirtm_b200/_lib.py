@@ -70,6 +70,7 @@ def lib():
          ctypes.POINTER(RtmTune), ctypes.POINTER(vp))
     _sig(L, "rtm_plan_destroy", c_int, vp)
     _sig(L, "rtm_plan_resident", c_int, vp)
+    _sig(L, "rtm_plan_resident_layout", c_int, vp, I32P)
     _sig(L, "rtm_plan_status", c_int, vp, I32P, vp)
     _sig(L, "rtm_plan_set_wait_limit", c_int, vp, c_int)
     _sig(L, "rtm_plan_pitch", c_int, vp)

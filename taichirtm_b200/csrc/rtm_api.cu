@@ -1208,6 +1208,15 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
 
 int rtm_plan_resident(const rtm_plan *p) { return p && p->res.layout >= 0 ? 1 : 0; }
 
+int rtm_plan_resident_layout(const rtm_plan *p, int32_t *layout) {
+    if (!p || !layout) return fail(RTM_E_ARG, "null argument");
+    if (p->res.layout < 0) return fail(RTM_E_STATE, "the plan streams its wavefield");
+    const ResLayout &l = RES_LAYOUTS[p->res.layout];
+    const int32_t v[5] = {l.rp, l.rs, l.warps, (int32_t)p->res.waves.size(), p->res.image_fits};
+    std::copy(v, v + 5, layout);
+    return RTM_OK;
+}
+
 int rtm_plan_set_wait_limit(rtm_plan *p, int polls) {
     if (!p) return fail(RTM_E_ARG, "null plan");
 #ifdef RTM_BOUNDS_CHECK

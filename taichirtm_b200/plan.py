@@ -96,6 +96,15 @@ class Plan:
         (rtm_plan_resident)."""
         return bool(_lib.lib().rtm_plan_resident(self.h))
 
+    def resident_layout(self):
+        """(rows per lane P-SV, SH, warps, launches per loop, images on the chip)
+        of a resident plan (rtm_plan_resident_layout), None for others."""
+        if not self.resident():
+            return None
+        out = np.zeros(5, np.int32)
+        check(_lib.lib().rtm_plan_resident_layout(self.h, _i32p(out)), "rtm_plan_resident_layout")
+        return tuple(out.tolist())
+
     def launch_count(self):
         return int(_lib.lib().rtm_plan_launch_count(self.h))
 

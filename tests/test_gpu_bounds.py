@@ -73,3 +73,14 @@ def test_kernels_stay_inside_their_buffers():
             f"sys.exit(pytest.main(['-x', '-q', '-p', 'no:cacheprovider'] + {tests!r}))")
     r = _child(code, timeout=1800)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+def test_resident_loops_stay_inside_their_buffers():
+    """The resident loops' tests, tile edges and several tile columns among them,
+    against the checking library."""
+    tests = ["tests/test_gpu_resident.py", "tests/test_gpu_resident_layouts.py"]
+    code = ("import sys, pytest; from taichirtm_b200 import _lib; "
+            "assert b'bounds-checking' in _lib.lib().rtm_version(); "
+            f"sys.exit(pytest.main(['-x', '-q', '-p', 'no:cacheprovider', '-k', 'not two_threads'] + {tests!r}))")
+    r = _child(code, timeout=1800)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
