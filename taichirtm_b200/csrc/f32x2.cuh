@@ -38,9 +38,6 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b, f2 neg_zero) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(neg_zero));
     return d;
 }
-__device__ __forceinline__ f2 f2_sel(bool lo, bool hi, f2 a, f2 b) {
-    return f2_pack(lo ? f2_lo(a) : f2_lo(b), hi ? f2_hi(a) : f2_hi(b));
-}
 
 // Two lanes of arithmetic on an f2: packed instructions, or two scalar ones (for
 // kernels that lose more to the even register pairs than packing saves).

@@ -93,21 +93,22 @@ struct ResParams {
 // surface mask).
 template <int MODE, int R, int NW>
 struct ResSmem {
+    static_assert(MODE == 1 || MODE == 2, "a tile is P-SV or SH");
     static constexpr int CELLS = NW * R * 32, ROWS = NW * R;
-    static constexpr int NC = ((MODE & 1) ? 2 : 0) + ((MODE & 2) ? 1 : 0);  // velocity components
+    static constexpr int NC = MODE == 1 ? 2 : 1;                     // velocity components
     static constexpr int IR = 0;                                     // P-SV (1/rho_u, 1/rho_w), 16 B
-    static constexpr int LM = IR + ((MODE & 1) ? CELLS * 16 : 0);    // (lam, 2 mu)
-    static constexpr int MY = LM + ((MODE & 1) ? CELLS * 16 : 0);    // SH (sdt myx, sdt myz)
-    static constexpr int XZ = MY + ((MODE & 2) ? CELLS * 16 : 0);    // sdt mxz, 8 B
-    static constexpr int IV = XZ + ((MODE & 1) ? CELLS * 8 : 0);     // 1/rho
-    static constexpr int C = IV + ((MODE & 2) ? CELLS * 8 : 0);      // sponge
+    static constexpr int LM = IR + (MODE == 1 ? CELLS * 16 : 0);    // (lam, 2 mu)
+    static constexpr int MY = LM + (MODE == 1 ? CELLS * 16 : 0);    // SH (sdt myx, sdt myz)
+    static constexpr int XZ = MY + (MODE == 2 ? CELLS * 16 : 0);    // sdt mxz, 8 B
+    static constexpr int IV = XZ + (MODE == 1 ? CELLS * 8 : 0);     // 1/rho
+    static constexpr int C = IV + (MODE == 2 ? CELLS * 8 : 0);      // sponge
     static constexpr int VEL = C + CELLS * 8;                        // [comp][warp + 1][lane]
     static constexpr int SIG = VEL + (NW + 2) * 32 * 8 * NC;         // xx, xz / yx
     // exchange: owned rows and lanes, floats and packets of a lane's pair, halo
     // packets of a tile (their values are staged over VEL and SIG, idle then)
     static constexpr int ORW = ROWS - 2 * RES_HALO, OLN = 32 - RES_HALO;
-    static constexpr int NF = ((MODE & 1) ? 10 : 0) + ((MODE & 2) ? 6 : 0), NP = (NF + 2) / 3;
-    static constexpr int NPAIR = MODE == 1 ? 3 : MODE == 2 ? 2 : 5;  // packets that carry a whole pair
+    static constexpr int NF = MODE == 1 ? 10 : 6, NP = (NF + 2) / 3;
+    static constexpr int NPAIR = MODE == 1 ? 3 : 2;                  // packets that carry a whole pair
     static constexpr int BOX = ORW * OLN * NP;
     static constexpr int STAGE = (2 * RES_HALO * 32 + ORW * RES_HALO) * NF * 4, ROWBUF = 2 * (NW + 2) * 32 * 8 * NC;
     static constexpr int INFO = VEL + ((STAGE > ROWBUF ? STAGE : ROWBUF) + 15) / 16 * 16;  // ResInfo
@@ -179,7 +180,7 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
 // registers per field (5 P-SV, 3 SH), the arithmetic of a row about 40 more.
 template <int MODE, int R, int NW>
 constexpr int res_ctas() {
-    constexpr int state = 2 * R * (((MODE & 1) ? 5 : 0) + ((MODE & 2) ? 3 : 0));
+    constexpr int state = 2 * R * (MODE == 1 ? 5 : 3);
     return (state <= 30 ? 32 : state <= 40 ? 24 : 16) / NW;
 }
 
@@ -188,10 +189,8 @@ extern __shared__ __align__(16) unsigned char res_smem_raw[];
 template <int DIR, int MODE, int R, int NW>
 __device__ __forceinline__ void resident_body(const ResParams &p) {
     using L = ResSmem<MODE, R, NW>;
-    constexpr bool PSV = (MODE & 1) != 0;
-    constexpr bool SH = (MODE & 2) != 0;
+    constexpr bool PSV = MODE == 1, SH = MODE == 2;
     constexpr int NC = L::NC;
-    constexpr int CV = PSV ? 2 : 0;  // v's place among the components
     constexpr int RT = L::ROWS;
     const int lane = threadIdx.x & 31;
     const int warp = __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0);  // known to be the same on every lane
@@ -437,12 +436,12 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
     auto publish_sig = [&]() {
         constexpr int r = DIR == 0 ? R - 1 : 0;
         if constexpr (PSV) { pub(L::SIG, 0, 0) = XX[r]; pub(L::SIG, 1, 0) = XZ[r]; }
-        if constexpr (SH) pub(L::SIG, CV, 0) = YX[r];
+        if constexpr (SH) pub(L::SIG, 0, 0) = YX[r];
     };
     auto publish_vel = [&]() {
         constexpr int r = DIR == 0 ? 0 : R - 1;
         if constexpr (PSV) { pub(L::VEL, 0, 0) = U[r]; pub(L::VEL, 1, 0) = W[r]; }
-        if constexpr (SH) pub(L::VEL, CV, 0) = V[r];
+        if constexpr (SH) pub(L::VEL, 0, 0) = V[r];
     };
     // An update of a row with edge cells: cells that are not interior keep their
     // value.  Their increment is cleared bitwise, so not even a NaN gets in.
@@ -457,7 +456,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         constexpr int D = DIR == 0 ? -1 : 1;
         [[maybe_unused]] f2 nxx = 0, nxz = 0, nyx = 0;  // the neighbouring warp's stress row
         if constexpr (PSV) { nxx = pub(L::SIG, 0, D); nxz = pub(L::SIG, 1, D); }
-        if constexpr (SH) nyx = pub(L::SIG, CV, D);
+        if constexpr (SH) nyx = pub(L::SIG, 0, D);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const int r = DIR == 0 ? k : R - 1 - k;
@@ -540,7 +539,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 add_at(U, row, c, scaled(0, ir.x, true));
                 add_at(W, row, c, scaled(1, ir.y, true));
             }
-            if constexpr (SH) add_at_v(V, row, c, scaled(CV, *reinterpret_cast<const f2 *>(c8 + L::IV + row * 256), false));
+            if constexpr (SH) add_at_v(V, row, c, scaled(0, *reinterpret_cast<const f2 *>(c8 + L::IV + row * 256), false));
         }
     };
     // Observed data by the table: one receiver per pair of cells at most.
@@ -556,7 +555,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 x = f2_add(x, f2_pack(have && !(t & 1) ? a : -0.0f, have && (t & 1) ? a : -0.0f));
             };
             if constexpr (PSV) { add(U[r], 0); add(W[r], 1); }
-            if constexpr (SH) add(V[r], CV);
+            if constexpr (SH) add(V[r], 0);
         }
     };
     // Stress update and absorbing (fm:369-419, bm:366-419); KIND as `kind`.
@@ -565,7 +564,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
         constexpr int D = DIR == 0 ? 1 : -1;
         [[maybe_unused]] f2 nu = 0, nw_ = 0, nv = 0;  // the neighbouring warp's velocity row
         if constexpr (PSV) { nu = pub(L::VEL, 0, D); nw_ = pub(L::VEL, 1, D); }
-        if constexpr (SH) nv = pub(L::VEL, CV, D);
+        if constexpr (SH) nv = pub(L::VEL, 0, D);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             // in the order in which row r's raw velocity is last read
@@ -701,7 +700,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 for (int r = 0; r < R; ++r) {
                     if (!(own >> r & 1)) continue;
                     if constexpr (PSV) { image(0, r, U[r]); image(1, r, W[r]); }
-                    if constexpr (SH) image(CV, r, V[r]);
+                    if constexpr (SH) image(0, r, V[r]);
                 }
                 return;
             }
@@ -757,7 +756,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
             if (!(own >> r & 1)) continue;
             auto get = [&](int comp, int c) { cp_async_vec<2>(reinterpret_cast<float *>(&s_img(comp, 2, r)), p.snap[c] + o + (long long)r * p.pitch); };
             if constexpr (PSV) { get(0, 0); get(1, 2); }
-            if constexpr (SH) get(CV, 1);
+            if constexpr (SH) get(0, 1);
         }
         cp_async_commit();
     };
@@ -777,7 +776,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 }
             };
             if constexpr (PSV) { move(0, 0); move(1, 2); }
-            if constexpr (SH) move(CV, 1);
+            if constexpr (SH) move(0, 1);
         }
     };
     // Finite check (fm:455-488, bm:417-450) of the owned cells.
@@ -850,7 +849,7 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 cp_async_vec<1>(s_val() + ((size_t)s * NC + comp) * p.max_inj + e, src);
             };
             if constexpr (PSV) { stage(0, 0); stage(1, 2); }
-            if constexpr (SH) stage(CV, 1);
+            if constexpr (SH) stage(0, 1);
         }
         cp_async_commit();
         if (blk > 0) {
@@ -867,19 +866,13 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                     if (!(own >> r & 1) || !(side || rr < 2 * RES_HALO || rr >= RT - 2 * RES_HALO)) continue;
                     uint4 *q = box + (size_t)blockIdx.x * p.box_stride + (rr - RES_HALO) * (L::NP * L::OLN) + ol;
                     if (!RTM_DBG_OK(q, 16) || !RTM_DBG_OK(q + (L::NP - 1) * L::OLN, 16)) continue;
-                    // packet k: pair k and one value of the pairs left over (L::place)
+                    // packet k: pair k and one value of the pairs left over
                     if constexpr (PSV) {
                         st_packet(q, U[r], f2_lo(W[r]), tag);
                         st_packet(q + L::OLN, XX[r], f2_hi(W[r]), tag);
                         st_packet(q + 2 * L::OLN, ZZ[r], f2_lo(XZ[r]), tag);
-                    }
-                    if constexpr (PSV && !SH) st_packet(q + 3 * L::OLN, 0ull, f2_hi(XZ[r]), tag);
-                    if constexpr (PSV && SH) {
-                        st_packet(q + 3 * L::OLN, V[r], f2_hi(XZ[r]), tag);
-                        st_packet(q + 4 * L::OLN, YX[r], f2_lo(YZ[r]), tag);
-                        st_packet(q + 5 * L::OLN, 0ull, f2_hi(YZ[r]), tag);
-                    }
-                    if constexpr (!PSV) {
+                        st_packet(q + 3 * L::OLN, 0ull, f2_hi(XZ[r]), tag);
+                    } else {
                         st_packet(q, V[r], f2_lo(YZ[r]), tag);
                         st_packet(q + L::OLN, YX[r], f2_hi(YZ[r]), tag);
                     }
@@ -993,15 +986,11 @@ __device__ __forceinline__ void resident_body(const ResParams &p) {
                 const bool get = (hl || hr) && ci && (in >> r & 1);
                 const int cell = hr ? (rr < RES_HALO ? rr : rr - L::ORW) * 32 + lane : slane + (rr - RES_HALO) * RES_HALO;
                 const unsigned q = sbase + cell * (L::NF * 4);
-                if constexpr (PSV && !SH) {
+                if constexpr (PSV) {
                     lds_if(U[r], q, get); lds_if(XX[r], q + 8, get); lds_if(ZZ[r], q + 16, get);
                     lds_if(W[r], q + 24, get); lds_if(XZ[r], q + 32, get);
                 }
-                if constexpr (PSV && SH) {
-                    lds_if(U[r], q, get); lds_if(XX[r], q + 8, get); lds_if(ZZ[r], q + 16, get); lds_if(V[r], q + 24, get);
-                    lds_if(YX[r], q + 32, get); lds_if(W[r], q + 40, get); lds_if(XZ[r], q + 48, get); lds_if(YZ[r], q + 56, get);
-                }
-                if constexpr (!PSV) { lds_if(V[r], q, get); lds_if(YX[r], q + 8, get); lds_if(YZ[r], q + 16, get); }
+                if constexpr (SH) { lds_if(V[r], q, get); lds_if(YX[r], q + 8, get); lds_if(YZ[r], q + 16, get); }
             }
             __syncthreads();
             publish_sig();

@@ -1722,8 +1722,11 @@ CkptOut ckpt_out(const rtm_plan *p, void *ckpt, int dtype, int c) {
     return o;
 }
 
-// Restore compressed slot c into the 5 FP32 fields `dst` (their pad rows and
-// pad columns are left as they are: zero).
+// Restore compressed slot c into the 5 FP32 fields `dst`: the interior rows, in the
+// columns that the strips cover (an even number, nz or more).  Pad rows and the left
+// pad columns are left as they are: callers whose streaming launches read them clear
+// them before; a resident launch reads only rows of the window and pairs of columns
+// that begin below nz.
 int ckpt_load(rtm_plan *p, const void *ckpt, int dtype, int c, float *const *dst, cudaStream_t s) {
     const CkptOut o = ckpt_out(p, const_cast<void *>(ckpt), dtype, c);
     CkptIn ci{};
