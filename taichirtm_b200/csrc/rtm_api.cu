@@ -1005,6 +1005,9 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     rtm_plan *p = new rtm_plan();
     p->g = g;
     p->nshots = nshots;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
     if (tune) {
         if (tune->vec == 1 || tune->vec == 2 || tune->vec == 4) p->vec = tune->vec;
         if (tune->rows > 0) p->rows = tune->rows;
@@ -1033,13 +1036,13 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
         p->vec = 2;
         p->tsteps = 2;
         p->rows = 24;
-        while (p->rows > 1 && rows_all / p->rows * strips < 148 * 16) p->rows /= 2;
+        while (p->rows > 1 && rows_all / p->rows * strips < sms * 16) p->rows /= 2;
         p->warps = 4;
         p->prefetch = p->rows >= 12 ? 3 : 1;
         // Long lists of tasks run fastest with 4 columns per lane, one warp per CTA
         // (14 windows of about 800 x 716, both wave types: 71 against 100 us per
         // step).  P-SV plans may be asked for an adjoint, which 2 columns suit.
-        if (g.modes != RTM_PSV && rows_all / 24 * ((g.nz + 119) / 120) >= 148 * 12) {
+        if (g.modes != RTM_PSV && rows_all / 24 * ((g.nz + 119) / 120) >= sms * 12) {
             p->vec = 4;
             p->rows = 24;
             p->warps = 1;
@@ -1129,12 +1132,7 @@ int rtm_plan_create(const rtm_grid *grid, int nshots, const rtm_shot *shots, con
     // together.  Any partition of a shot's rows into tasks gives the same
     // results; a half keeps its parent's no-source / no-receiver flags, which
     // hold for any sub-range of rows.
-    {
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            sms = 148;
-        split_tail(work, tail_split_tasks(work.size(), sms));
-    }
+    split_tail(work, tail_split_tasks(work.size(), sms));
     p->n_work = (int)work.size();
     p->state_floats = (size_t)state_rows * p->pitch;
     const size_t mat_floats = (size_t)(g.nx + 2) * p->pitch;
