@@ -545,7 +545,7 @@ def main():
             o0 = sum(len(x.src) for x in shots[:s])
             r0 = sum(len(x.rec) for x in shots[:s])
             one = BatchedRTM(mu_m, lam_m, rho_m, survey.dx, survey.dz, survey.fs, nt, survey.fw, sub,
-                             modes=PSV, tune="auto", device=dev)  # each one-shot plan tuned for itself
+                             modes=PSV, tune="auto", device=dev)  # each one-shot plan resident or tuned for itself
             shapes.append({k: v for k, v in one.tune.items() if k != "graphs"})
             w1 = wav[:, o0:o0 + len(sub[0].src)].contiguous()
             o1 = obs[:, r0:r0 + len(sub[0].rec)].contiguous()
@@ -560,7 +560,7 @@ def main():
             one.close()
         return dict(shots_per_s=round(nplain / (t_sum / 1000.0), 3), launch_shapes=shapes,
                     sample=f"shots 0..{nplain - 1} migrated one shot per plan (one shot per launch), "
-                           "each plan with its own autotuned launch shape")
+                           "each plan with tune=\"auto\": resident on the chip (launch shape {}) or its own autotuned shape")
 
     # the plain path, checkpointed RTM and gradient legs are one-GPU
     # comparisons: run at N = 1 only, so an N-GPU run holds its GPUs for the

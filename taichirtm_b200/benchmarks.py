@@ -156,7 +156,7 @@ def _plain_gradient(sv, shots, wav, obs, m0, K, nt, dev, nplain):
         one.close()
     return dict(shots_per_s=round(nplain / (t_sum / 1000.0), 3), launch_shapes=shapes,
                 sample=f"shots 0..{nplain - 1}, one shot per problem (one shot per launch), "
-                       "each with its own autotuned launch shape")
+                       "each with its own autotuned launch shape ({}: the library's choice)")
 
 
 def gradient_leg(nt=3000, steps=3, warmup=1, nplain=2, with_reference_image=False):

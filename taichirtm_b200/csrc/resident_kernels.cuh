@@ -177,7 +177,9 @@ __device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long lon
 }
 
 // CTAs per SM that the register budget is cut for: the wavefield takes 2 R
-// registers per field (5 P-SV, 3 SH), the arithmetic of a row about 40 more.
+// registers per field (5 P-SV, 3 SH), the arithmetic of a row about 40 more.  At
+// these budgets most kernels spill some (the table of layouts in rtm_api.cu has
+// the bytes).
 template <int MODE, int R, int NW>
 constexpr int res_ctas() {
     constexpr int state = 2 * R * (MODE == 1 ? 5 : 3);

@@ -58,8 +58,8 @@ int dalloc(T **p, size_t n) {
 }
 
 // Device buffers that live and die together, in one allocation.  A plan has about
-// 45 of them; one by one, their cudaMalloc and cudaFree calls took 8.8 and 2.5 ms
-// (395 x 395, both wave types), most of a short one-shot run.
+// 45 of them; one by one, making and destroying one took 6.9 and 5.3 ms (395 x 395,
+// both wave types), most of a short one-shot run; together 0.9 and 0.6.
 struct Slab {
     std::vector<std::pair<void **, size_t>> want;
     void *base = nullptr;
@@ -655,7 +655,10 @@ int read_status(rtm_plan *p, int32_t *flags, cudaStream_t s) {
 // recompute a smaller share of halo.  Layouts that another one beats at every
 // size are not built (P-SV R 4 x 8 warps: 432 CTAs hold 581,000 cells at 3.7 us,
 // R 6 x 8: 288 hold 645,000 at 3.3; R 3 x 16 is 5 % behind R 6 x 8; R 7 and 8
-// spill: 188 / 163 and 139 Gcell/s against 190).
+// spill so much that they run at 188 / 163 and 139 Gcell/s against 190).  The ones
+// built spill a little, too, at these registers (bytes stored, forward / backward):
+// P-SV R 2 x 8 60 / 184 and R 6 x 8 256 / 188, SH 0 to 44, both wave types 76 / 300
+// and 260 / 220; P-SV R 2 x 12 0 / 72.
 struct ResLayout {
     int mode, rp, rs, warps;
     float us[4];
