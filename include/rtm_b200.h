@@ -238,7 +238,8 @@ int rtm_forward_checkpointed(rtm_plan *plan, const float *wavelets, float *seis,
  * the reverse sweep run steps in pairs; the gradient is bit-identical.
  * Its scratch (ckpt_every + 3 states plus the gradient sums) is allocated on
  * the first call and kept by the plan, grown when a later call needs more,
- * and freed by rtm_plan_destroy; rtm_backward_checkpointed shares it. */
+ * and freed by rtm_plan_destroy; rtm_backward_checkpointed and
+ * rtm_backward_normalized (one FP64 value per shot cell) share it. */
 int rtm_adjoint(rtm_plan *plan, const float *wavelets, const float *resid, int ckpt_every,
                 int ckpt_dtype, const void *ckpt, double *grad, float *grad_wavelet,
                 rtm_stream_t stream);
